@@ -10,16 +10,15 @@
 // adjacent merged), then one of two kernels runs:
 //  * the innermost axis is preserved -> a row-gather copy in 16-byte vectors where the
 //    row length and pointers allow (every warp reads and writes whole contiguous runs);
-//  * otherwise a tiled transpose between the input's fastest axis and the output's
-//    fastest axis, so both the HBM reads and the HBM writes are coalesced; all remaining
-//    axes are batch axes decomposed per tile.  For 1-, 2- and 4-byte elements, when the
-//    input strides allow a tensor map (16-byte multiples, at most 3 batch axes), the
-//    tiles are staged by TMA: a persistent CTA double-buffers (128 bytes of the input's
-//    fastest axis) x 64 tiles into shared memory with cp.async.bulk.tensor
+//  * otherwise a tiled transpose between the input's fastest axes and the output's
+//    fastest axes, so both the HBM reads and the HBM writes are coalesced; all remaining
+//    axes are batch axes decomposed per tile (k_tile_transpose).  For 1- and 2-byte
+//    elements, when the input strides allow a tensor map (16-byte multiples, at most 3
+//    batch axes), the tiles are staged by TMA: a persistent CTA double-buffers (128 bytes
+//    of the input's fastest axis) x 128 tiles into shared memory with cp.async.bulk.tensor
 //    (SWIZZLE_128B, so the column reads of the transpose spread over the banks) and
-//    writes 16-byte vectors along the output's fastest axis.  Otherwise (8-byte
-//    elements, short output axes, other strides) a 32x32-element shared-memory tile
-//    kernel runs.
+//    writes 16-byte vectors along the output's fastest axis.  A short output axis (< 16)
+//    under a long input axis has a staged kernel of its own.
 // No per-call allocation or host<->device copy of stride vectors: the reduced
 // geometry travels as kernel parameters (the reference mallocs and copies two
 // stride arrays per call, cuMovemem_gpu.cu:139-152).
@@ -91,91 +90,240 @@ __global__ void __launch_bounds__(256) k_row_gather(const U *__restrict__ src, U
 
 // ---------------------------------------------------------------- tiled transpose
 // Input fastest axis "a" (new position pa), output fastest axis "b" (old axis with
-// input stride sb).  Tile: 32 (b) x 32 (a) elements; block 32 x 8 threads.
+// input stride sb), for the staged kernel below.
 struct TransGeom {
   int nbatch_dims;
   int64_t na, nb;           // sizes of axes a and b
   int64_t out_stride_a;     // output stride of axis a
   int64_t in_stride_b;      // input stride of axis b
-  int64_t tiles_a, tiles_b; // tile counts
   int64_t batch;            // number of batch points
   int64_t bshape[kMaxRank]; // batch axes (new order, row-major over them)
   int64_t bin[kMaxRank];    // their input strides
   int64_t bout[kMaxRank];   // their output strides
 };
 
-// IT: the integer type of the tile and batch index arithmetic (32-bit when the tile count
-// and every batch axis fit, which turns the per-tile divisions from 64-bit software routines
-// into 32-bit ones); element offsets stay 64-bit.
-template <typename T, typename IT>
-__global__ void __launch_bounds__(256) k_transpose(const T *__restrict__ src, T *__restrict__ dst,
-                                                   TransGeom g) {
-  __shared__ T tile[32][33];
-  const IT tiles_a = (IT)g.tiles_a;
-  const IT ntile = (IT)(g.tiles_a * g.tiles_b);
-  const IT total = (IT)(g.tiles_a * g.tiles_b * g.batch);
-  for (IT t = blockIdx.x; t < total; t += gridDim.x) {
-    const IT bidx = t / ntile;
-    const IT tt = t - bidx * ntile;
-    const IT tb = tt / tiles_a;
-    const IT ta = tt - tb * tiles_a;
-    int64_t in_off = 0, out_off = 0;
-    IT r = bidx;
-    for (int i = g.nbatch_dims - 1; i >= 0; --i) {
-      const IT d = (IT)g.bshape[i];
-      const IT q = r / d;
-      const IT c = r - q * d;
-      in_off += (int64_t)c * g.bin[i];
-      out_off += (int64_t)c * g.bout[i];
-      r = q;
-    }
-    const int64_t a0 = (int64_t)ta * 32, b0 = (int64_t)tb * 32;
-    // read: rows of b, contiguous along a
-    const int64_t ia = a0 + threadIdx.x;
-#pragma unroll
-    for (int j = 0; j < 32; j += 8) {
-      int64_t ib = b0 + threadIdx.y + j;
-      if (ia < g.na && ib < g.nb) tile[threadIdx.y + j][threadIdx.x] = src[in_off + ib * g.in_stride_b + ia];
-    }
-    __syncthreads();
-    // write: rows of a, contiguous along b
-    const int64_t ob = b0 + threadIdx.x;
-#pragma unroll
-    for (int j = 0; j < 32; j += 8) {
-      int64_t oa = a0 + threadIdx.y + j;
-      if (oa < g.na && ob < g.nb) dst[out_off + oa * g.out_stride_a + ob] = tile[threadIdx.x][threadIdx.y + j];
+// General tiled transpose, any element size, strides and extents.  The reduced axes fall into
+// three groups: A, contiguous in the input (the input's fastest axis and, while the product is
+// below the wanted run, the axes next to it in the input), B, contiguous in the output (the
+// output's fastest axis and its neighbours likewise), and the batch axes.  A CTA moves one tile
+// of TA x TB elements: it reads runs of TA along A, stages them in shared memory and writes
+// runs of TB along B.  Grouping axes keeps the runs long when the last axes are short (a site
+// tensor's physical legs, a 37-element leg), and the tile's shape (powers of two, TA * TB = CAP)
+// follows the groups' extents, so few lanes idle on them.
+// These kernels are bound by instruction issue before HBM (a 32-lane access moves 32 elements of
+// a narrow type only), so a tile's shape is a compile-time constant: a row costs one offset and
+// one 64-bit multiply-add, an element its load, its store and the shared-memory round trip.  All
+// loads of a thread (CAP / 256 elements) are issued before the first store.  Element accesses
+// throughout: nothing is asked of the alignment of rows, strides or base pointers.
+// Measured (TB/s read + written), the 32 x 32 kernel this replaced -> this one: f64
+// [2048,3,3,2048] reversed 5.9 -> 6.4, [2047,3,3,2045] 5.3 -> 6.1, [4000000,5] 1.6 -> 6.2; f32
+// [2047,3,3,2045] 3.4 -> 5.5, [1021,3,37,509] (3,1,0,2) 1.8 -> 4.5, and the aligned
+// [2048,3,3,2048], which a TMA-staged kernel moved at 4.7, 6.1; int16 ragged 0.9-1.8 -> 3.6-3.9.
+constexpr int TILE_THREADS = 256;
+// elements per tile, by measurement ([2048,3,3,2048] reversed): f64 1024 / 2048 elements 110 / 94
+// us, f32 2048 / 4096 63 / 49 us; 16-byte elements and small tensors 1024 (four loads per thread)
+constexpr int TILE_SMALL = 1024;
+constexpr int tile_cap(int es) { return es == 1 ? 8192 : es <= 4 ? 4096 : es == 8 ? 2048 : 1024; }
+constexpr int TILE_TA_MIN = 2, TILE_TA_MAX = 1024;  // tile widths along A (TB = CAP / TA likewise >= 2)
+// staged row pitch in elements: an odd number of 32-bit words (wider types: odd), so that the
+// column reads of consecutive b fall on different banks
+constexpr int tile_pitch(int es, int ta) {
+  return es >= 4 ? (ta | 1) : es == 2 ? (ta % 4 == 0 ? ta + 2 : ta) : (ta % 8 == 0 ? ta + 4 : ta);
+}
+
+template <int R, typename IT>
+struct TilePerm {
+  int64_t src, dst;            // element offsets of the permuted block
+  IT ext[R], ins[R], outs[R];  // axes: A group (innermost first), B group (innermost first), batch
+  IT na, nb;                   // extents of the groups
+  IT tiles_a, tiles_b;
+  int8_t n_a, n_b, n_x;        // axes per group
+  int8_t log_ta;               // the tile's width along A
+};
+
+// offset of index x of the group whose axes are k0 .. k0 + n - 1 (innermost first)
+template <int R, typename IT>
+__device__ __forceinline__ IT group_offset(const TilePerm<R, IT> &g, const IT *st, int k0, int n, IT x) {
+  IT o = 0;
+  for (int k = k0; k + 1 < k0 + n; ++k) {
+    const IT d = g.ext[k];
+    const IT q = x / d;
+    o += (x - q * d) * st[k];
+    x = q;
+  }
+  return o + x * st[k0 + n - 1];
+}
+
+template <typename T, int CAP, int TA, typename IT>
+struct TileSmem {
+  static constexpr int TB = CAP / TA;
+  static constexpr int PITCH = tile_pitch((int)sizeof(T), TA);
+  T tile[TB * PITCH];
+  IT off[TA + TB];  // [0, TA): output offsets of the tile's a, [TA, TA + TB): input offsets of its b
+};
+
+template <typename T, int CAP, int TA, int R, typename IT>
+__device__ __forceinline__ void tile_transpose(const TilePerm<R, IT> &g, IT t, const T *__restrict__ src,
+                                               T *__restrict__ dst, void *smem) {
+  using SM = TileSmem<T, CAP, TA, IT>;
+  constexpr int TB = SM::TB, PITCH = SM::PITCH;
+  constexpr int WA = TA < 32 ? TA : 32, HA = TA / WA, RA = TILE_THREADS / WA;  // reading: lanes along A, rows of b
+  constexpr int WB = TB < 32 ? TB : 32, HB = TB / WB, RB = TILE_THREADS / WB;  // writing: lanes along B, rows of a
+  constexpr int NRA = TB / RA > 0 ? TB / RA : 1, NRB = TA / RB > 0 ? TA / RB : 1;
+  static_assert(NRA * HA * TILE_THREADS >= CAP && NRB * HB * TILE_THREADS >= CAP, "tile coverage");
+  SM &sm = *reinterpret_cast<SM *>(smem);
+  const int tid = threadIdx.x;
+  IT r = t / g.tiles_a;
+  const IT a0 = (t - r * g.tiles_a) * (IT)TA;
+  const IT q = r / g.tiles_b;
+  const IT b0 = (r - q * g.tiles_b) * (IT)TB;
+  r = q;
+  IT in_off = a0, out_off = b0;
+  for (int i = 0; i < g.n_x; ++i) {
+    const int k = g.n_a + g.n_b + i;
+    const IT d = g.ext[k];
+    const IT qq = i + 1 < g.n_x ? r / d : 0;
+    const IT c = r - qq * d;
+    in_off += c * g.ins[k];
+    out_off += c * g.outs[k];
+    r = qq;
+  }
+  const int ca = (int)(g.na - a0 < (IT)TA ? g.na - a0 : (IT)TA);
+  const int cb = (int)(g.nb - b0 < (IT)TB ? g.nb - b0 : (IT)TB);
+  const bool one_a = g.n_a == 1, one_b = g.n_b == 1;  // single axes: offsets are multiples of one stride
+  const IT sa = g.outs[0], sb = g.ins[g.n_a];
+  if (!(one_a && one_b)) {
+    for (int i = tid; i < TA + TB; i += TILE_THREADS) {
+      if (i < TA) sm.off[i] = one_a ? 0 : group_offset(g, g.outs, 0, g.n_a, (IT)(a0 + (IT)i));
+      else sm.off[i] = one_b ? 0 : group_offset(g, g.ins, g.n_a, g.n_b, (IT)(b0 + (IT)(i - TA)));
     }
     __syncthreads();
   }
+  {
+    const int lane = tid % WA, row0 = tid / WA;
+    const T *s = src + g.src + (int64_t)in_off + lane;
+    T v[NRA][HA];
+#pragma unroll
+    for (int i = 0; i < NRA; ++i) {
+      const int b = row0 + i * RA;
+      const IT o = one_b ? (b0 + (IT)b) * sb : sm.off[TA + (TB % RA == 0 ? b : b % TB)];
+#pragma unroll
+      for (int h = 0; h < HA; ++h)
+        if (b < cb && lane + h * WA < ca) v[i][h] = s[(int64_t)o + h * WA];
+    }
+#pragma unroll
+    for (int i = 0; i < NRA; ++i) {
+      const int b = row0 + i * RA;
+#pragma unroll
+      for (int h = 0; h < HA; ++h)
+        if (b < cb && lane + h * WA < ca) sm.tile[b * PITCH + lane + h * WA] = v[i][h];
+    }
+  }
+  __syncthreads();
+  {
+    const int lane = tid % WB, row0 = tid / WB;
+    T *o = dst + g.dst + (int64_t)out_off + lane;
+#pragma unroll
+    for (int i = 0; i < NRB; ++i) {
+      const int a = row0 + i * RB;
+      const IT oo = one_a ? (a0 + (IT)a) * sa : sm.off[TA % RB == 0 ? a : a % TA];
+#pragma unroll
+      for (int h = 0; h < HB; ++h)
+        if (a < ca && lane + h * WB < cb) o[(int64_t)oo + h * WB] = sm.tile[(lane + h * WB) * PITCH + a];
+    }
+  }
 }
 
-// Short output axis (nb < 16): one thread per (batch point, a) writes the nb consecutive
-// output elements of its row, reading them at input stride in_stride_b; the reads of a
-// warp are coalesced along a and the writes are contiguous runs.
-template <typename T>
-__global__ void __launch_bounds__(256) k_transpose_short(const T *__restrict__ src, T *__restrict__ dst, TransGeom g) {
-  const int64_t rows = g.na * g.batch;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rows; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t bidx = t / g.na;
-    const int64_t ia = t - bidx * g.na;
-    int64_t in_off = 0, out_off = 0;
-    for (int i = g.nbatch_dims - 1; i >= 0; --i) {
-      const int64_t d = g.bshape[i];
-      const int64_t q = bidx / d;
-      const int64_t c = bidx - q * d;
-      in_off += c * g.bin[i];
-      out_off += c * g.bout[i];
-      bidx = q;
+template <typename T, int CAP, int TA, typename IT>
+__global__ void __launch_bounds__(TILE_THREADS) k_tile_transpose(const T *__restrict__ src, T *__restrict__ dst,
+                                                                 const __grid_constant__ TilePerm<kMaxRank, IT> g,
+                                                                 int64_t ntiles) {
+  __shared__ __align__(16) unsigned char smem[sizeof(TileSmem<T, CAP, TA, IT>)];
+  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    tile_transpose<T, CAP, TA>(g, (IT)t, src, dst, smem);
+    __syncthreads();  // the next tile reuses the stage and the offsets
+  }
+}
+
+// Geometry of a reduced permutation whose innermost axis moves (reduce_perm's axes; strides in
+// elements).  Groups stop growing at `want` elements.  Returns the number of tiles of `cap`
+// elements.
+template <int R, typename IT>
+static int64_t tile_geometry(int es, int cap, int want, int r, const int64_t *rshape, const int *rmap, const int64_t *in_stride,
+                             const int64_t *out_stride_of_old, TilePerm<R, IT> &g) {
+  const int a = r - 1, b = rmap[r - 1];
+  bool used[kMaxRank] = {false};
+  int order[kMaxRank], n = 0;
+  int grp_b[kMaxRank], nb = 0;
+  int64_t eb = rshape[b], ea = rshape[a];
+  grp_b[nb++] = b;
+  used[b] = used[a] = true;
+  for (int i = r - 2; i >= 0 && rmap[i] != a && eb < want; --i) {  // output neighbours of b
+    grp_b[nb++] = rmap[i];
+    used[rmap[i]] = true;
+    eb *= rshape[rmap[i]];
+  }
+  order[n++] = a;
+  for (int j = r - 2; j >= 0 && !used[j] && ea < want; --j) {  // input neighbours of a
+    order[n++] = j;
+    used[j] = true;
+    ea *= rshape[j];
+  }
+  g.n_a = (int8_t)n;
+  for (int i = 0; i < nb; ++i) order[n++] = grp_b[i];
+  g.n_b = (int8_t)nb;
+  int64_t batch = 1;
+  for (int i = r - 1; i >= 0; --i)
+    if (!used[rmap[i]]) {
+      order[n++] = rmap[i];
+      batch *= rshape[rmap[i]];
     }
-    const T *s = src + in_off + ia;
-    T *o = dst + out_off + ia * g.out_stride_a;
-    T v[16];
-#pragma unroll
-    for (int b = 0; b < 16; ++b)
-      if (b < g.nb) v[b] = s[b * g.in_stride_b];
-#pragma unroll
-    for (int b = 0; b < 16; ++b)
-      if (b < g.nb) o[b] = v[b];
+  g.n_x = (int8_t)(n - g.n_a - g.n_b);
+  for (int k = 0; k < n; ++k) {
+    g.ext[k] = (IT)rshape[order[k]];
+    g.ins[k] = (IT)in_stride[order[k]];
+    g.outs[k] = (IT)out_stride_of_old[order[k]];
+  }
+  g.na = (IT)ea;
+  g.nb = (IT)eb;
+  // the width with the fewest tiles among those that keep runs of 64 bytes (or the whole group)
+  // on both sides; among equals the squarest tile
+  int64_t best = -1, best_skew = 0;
+  const int64_t least = std::max(2, 64 / es);
+  for (int l = 1; (1 << l) <= TILE_TA_MAX; ++l) {
+    const int64_t ta = (int64_t)1 << l, tb = cap / ta;
+    if (ta < TILE_TA_MIN || tb < TILE_TA_MIN || tb > TILE_TA_MAX) continue;
+    const bool keeps = ta >= std::min<int64_t>(ea, least) && tb >= std::min<int64_t>(eb, least);
+    const int64_t tiles = ((ea + ta - 1) / ta) * ((eb + tb - 1) / tb) + (keeps ? 0 : (int64_t)1 << 60);
+    const int64_t skew = std::max(ta, tb) / std::min(ta, tb);
+    if (best < 0 || tiles < best || (tiles == best && skew < best_skew)) {
+      best = tiles;
+      best_skew = skew;
+      g.log_ta = (int8_t)l;
+    }
+  }
+  const int64_t ta = (int64_t)1 << g.log_ta, tb = cap / ta;
+  const int64_t tiles_a = (ea + ta - 1) / ta, tiles_b = (eb + tb - 1) / tb;
+  g.tiles_a = (IT)tiles_a;
+  g.tiles_b = (IT)tiles_b;
+  return tiles_a * tiles_b * batch;
+}
+
+template <typename T, int CAP, typename IT>
+static void launch_tile(const void *src, void *dst, const TilePerm<kMaxRank, IT> &g, int64_t ntiles, cudaStream_t st) {
+  const unsigned grid = (unsigned)std::min<int64_t>(ntiles, (int64_t)1 << 30);
+  auto go = [&](auto kern) { kern<<<grid, TILE_THREADS, 0, st>>>((const T *)src, (T *)dst, g, ntiles); };
+  switch (g.log_ta) {
+    case 1: if constexpr (CAP / 2 <= TILE_TA_MAX) go(k_tile_transpose<T, CAP, 2, IT>); break;
+    case 2: if constexpr (CAP / 4 <= TILE_TA_MAX) go(k_tile_transpose<T, CAP, 4, IT>); break;
+    case 3: if constexpr (CAP / 8 <= TILE_TA_MAX) go(k_tile_transpose<T, CAP, 8, IT>); break;
+    case 4: if constexpr (CAP / 16 <= TILE_TA_MAX) go(k_tile_transpose<T, CAP, 16, IT>); break;
+    case 5: go(k_tile_transpose<T, CAP, 32, IT>); break;
+    case 6: go(k_tile_transpose<T, CAP, 64, IT>); break;
+    case 7: go(k_tile_transpose<T, CAP, 128, IT>); break;
+    case 8: go(k_tile_transpose<T, CAP, 256, IT>); break;
+    case 9: go(k_tile_transpose<T, CAP, 512, IT>); break;
+    default: if constexpr (CAP > 1024) go(k_tile_transpose<T, CAP, 1024, IT>); break;
   }
 }
 
@@ -291,14 +439,13 @@ static int sm_count() {
 }
 
 // ---------------------------------------------------------------- TMA-staged transpose
-// Tile: TA = 128 / ES elements of axis a (one 128-byte swizzle row) x TB = tma_tb(ES) of axis b.
+// Tile: TA = 128 / ES elements of axis a (one 128-byte swizzle row) x TB = 128 of axis b.
 // The tensor map views the input as [batch2][batch1][batch0][b][a] (a fastest); the
 // shared-memory image of a box row b is 128 bytes whose 16-byte chunks are XOR-swizzled
 // with (b & 7).  The 256 threads write the tile as 16-byte output vectors (16 / ES
 // consecutive b of one a), TA * TB * ES / 4096 of them each.
-// b rows per staged tile: 128 for 1- and 2-byte elements (16 KB tiles; int16 4.37 -> 4.83 TB/s
-// against 64 rows), 64 for 4-byte ones (128 rows: f32 4.56 -> 4.30 TB/s)
-constexpr int tma_tb(int es) { return es <= 2 ? 128 : 64; }
+// b rows per staged tile: 16 KB tiles (int16 4.37 -> 4.83 TB/s against 64 rows)
+constexpr int TMA_TB = 128;
 constexpr int TMA_THREADS = 256;
 constexpr long long TMA_SPIN = 1ll << 26;  // mbarrier probes before giving up
 
@@ -338,7 +485,6 @@ template <int ES, typename IT>
 __global__ void __launch_bounds__(TMA_THREADS) k_transpose_tma(const __grid_constant__ CUtensorMap in_map,
                                                               uint8_t *__restrict__ dst, TmaGeom g) {
   constexpr int TA = 128 / ES;
-  constexpr int TMA_TB = tma_tb(ES);
   constexpr int TILE = TMA_TB * 128;                   // bytes per staged tile
   constexpr int VEC = 16 / ES;                         // elements per output vector
   constexpr int CHUNKS = TMA_TB / VEC;                 // output vectors per a (along b)
@@ -496,7 +642,6 @@ template <int ES>
 static bool try_transpose_tma(const void *src, void *dst, int r, const int64_t *rshape, const int *rmap,
                               const int64_t *in_stride, const int64_t *out_stride, cudaStream_t st, ctn_status *res) {
   constexpr int TA = 128 / ES;
-  constexpr int TMA_TB = tma_tb(ES);
   const int a = r - 1, b = rmap[r - 1];
   if (r - 2 > 3) return false;
   int64_t nel = 1;
@@ -539,10 +684,7 @@ static bool try_transpose_tma(const void *src, void *dst, int r, const int64_t *
   CUtensorMap map;
   const cuuint32_t box[5] = {(cuuint32_t)TA, (cuuint32_t)TMA_TB, 1, 1, 1};
   const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  const CUtensorMapDataType dt = ES == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
-                                 : ES == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16
-                                 : ES == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32
-                                           : CU_TENSOR_MAP_DATA_TYPE_UINT64;
+  const CUtensorMapDataType dt = ES == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16;
   const EncodeTiledFn enc = encode_tiled();
   if (!enc) return false;
   if (enc(&map, dt, 5, const_cast<void *>(src), dims, strides, box, estr,
@@ -693,54 +835,62 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
     CTN_CHECK_LAUNCH();
     return CTN_OK;
   }
-  // TMA staging pays for 1-, 2- and 4-byte elements (f32 4.3 vs 2.9 TB/s, 16-bit 3.0 vs 1.5 TB/s
-  // on a 512 MB transpose); for 8-byte elements the 32x32 register tile is faster (4.9 vs 4.3
-  // TB/s), and a short output axis (< 16) wastes most of a staged tile
-  if (ES <= 4 && rshape[rmap[r - 1]] >= 16) {
+  // TMA staging pays for 1- and 2-byte elements ([2048,3,3,2048] reversed: int16 31 us against 38
+  // us in element accesses, bool 17 against 35); for 4-byte elements the element tiles are faster
+  // (49 against 64 us), and a short output axis (< 16) wastes most of a staged tile
+  if (ES <= 2 && rshape[rmap[r - 1]] >= 16) {
     ctn_status res = CTN_OK;
-    if (try_transpose_tma<(ES <= 4 ? ES : 4)>(src, dst, r, rshape, rmap, in_stride, out_stride, st, &res)) return res;
+    if (try_transpose_tma<(ES <= 2 ? ES : 2)>(src, dst, r, rshape, rmap, in_stride, out_stride, st, &res)) return res;
   }
-  TransGeom g;
   const int a = r - 1;        // input fastest (old axis)
   const int b = rmap[r - 1];  // old axis that is output fastest
-  int pa = 0;
-  for (int i = 0; i < r; ++i)
-    if (rmap[i] == a) pa = i;
-  g.na = rshape[a];
-  g.nb = rshape[b];
-  g.out_stride_a = out_stride[pa];
-  g.in_stride_b = in_stride[b];
-  g.tiles_a = (g.na + 31) / 32;
-  g.tiles_b = (g.nb + 31) / 32;
-  g.nbatch_dims = 0;
-  g.batch = 1;
-  for (int i = 0; i < r; ++i) {
-    const int j = rmap[i];
-    if (j == a || j == b) continue;
-    g.bshape[g.nbatch_dims] = rshape[j];
-    g.bin[g.nbatch_dims] = in_stride[j];
-    g.bout[g.nbatch_dims] = out_stride[i];
-    g.nbatch_dims++;
-    g.batch *= rshape[j];
-  }
-  if (g.nb < 16) {
+  if (rshape[b] < 16 && rshape[a] >= STAGED_THREADS) {
+    TransGeom g;
+    int pa = 0;
+    for (int i = 0; i < r; ++i)
+      if (rmap[i] == a) pa = i;
+    g.na = rshape[a];
+    g.nb = rshape[b];
+    g.out_stride_a = out_stride[pa];
+    g.in_stride_b = in_stride[b];
+    g.nbatch_dims = 0;
+    g.batch = 1;
+    for (int i = 0; i < r; ++i) {
+      const int j = rmap[i];
+      if (j == a || j == b) continue;
+      g.bshape[g.nbatch_dims] = rshape[j];
+      g.bin[g.nbatch_dims] = in_stride[j];
+      g.bout[g.nbatch_dims] = out_stride[i];
+      g.nbatch_dims++;
+      g.batch *= rshape[j];
+    }
     if (launch_staged<T>(src, dst, g, nsm, st)) {
       CTN_CHECK_LAUNCH();
       return CTN_OK;
     }
-    const int64_t rows = g.na * g.batch;
-    const int64_t blocks = std::min<int64_t>((rows + 255) / 256, (int64_t)nsm * 16);
-    k_transpose_short<T><<<(unsigned)blocks, 256, 0, st>>>((const T *)src, (T *)dst, g);
-    CTN_CHECK_LAUNCH();
-    return CTN_OK;
   }
-  const int64_t total = g.tiles_a * g.tiles_b * g.batch;
-  const int64_t blocks = std::min<int64_t>(total, (int64_t)nsm * 32);
-  // 32-bit tile arithmetic when the loop variable cannot pass 2^32 (t < total + grid)
-  if (total + blocks < ((int64_t)1 << 32))
-    k_transpose<T, uint32_t><<<(unsigned)blocks, dim3(32, 8), 0, st>>>((const T *)src, (T *)dst, g);
-  else
-    k_transpose<T, int64_t><<<(unsigned)blocks, dim3(32, 8), 0, st>>>((const T *)src, (T *)dst, g);
+  int64_t out_stride_of_old[kMaxRank];
+  for (int i = 0; i < r; ++i) out_stride_of_old[rmap[i]] = out_stride[i];
+  constexpr int WANT = ES == 1 ? 128 : 64;
+  // 32-bit index arithmetic (a division costs several times less) when every offset fits
+  if (n < ((int64_t)1 << 31)) {
+    TilePerm<kMaxRank, uint32_t> g;
+    g.src = g.dst = 0;
+    int64_t ntiles = tile_geometry(ES, tile_cap(ES), WANT, r, rshape, rmap, in_stride, out_stride_of_old, g);
+    // fewer than two tiles per SM: the latency of one tile is all there is, so smaller tiles, and
+    // axes joined only where a group would be very short (a joined group needs an offset table)
+    if (ntiles < 2 * nsm) {
+      ntiles = tile_geometry(ES, TILE_SMALL, 16, r, rshape, rmap, in_stride, out_stride_of_old, g);
+      launch_tile<T, TILE_SMALL>(src, dst, g, ntiles, st);
+    } else {
+      launch_tile<T, tile_cap(ES)>(src, dst, g, ntiles, st);
+    }
+  } else {
+    TilePerm<kMaxRank, uint64_t> g;
+    g.src = g.dst = 0;
+    const int64_t ntiles = tile_geometry(ES, tile_cap(ES), WANT, r, rshape, rmap, in_stride, out_stride_of_old, g);
+    launch_tile<T, tile_cap(ES)>(src, dst, g, ntiles, st);
+  }
   CTN_CHECK_LAUNCH();
   return CTN_OK;
 }
