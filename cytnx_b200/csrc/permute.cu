@@ -34,13 +34,6 @@ namespace ctn {
 
 constexpr int kMaxRank = 16;
 
-struct PermGeom {
-  int rank;                   // reduced rank (>= 2 here)
-  int64_t n;                  // total elements
-  int64_t out_shape[kMaxRank];    // new shape (reduced)
-  int64_t in_stride_of_out[kMaxRank];  // input stride of the old axis at new position i
-};
-
 struct alignas(16) U128 {
   uint64_t a, b;
 };
@@ -58,34 +51,104 @@ struct VecT<8> { using T = uint64_t; };
 template <>
 struct VecT<16> { using T = U128; };
 
-// ---------------------------------------------------------------- row gather
-// The last new axis equals the last old axis.  Each "unit" is V bytes; the row of
-// the innermost axis holds row_units units.  For out unit u: row = u / row_units,
-// col = u % row_units; the row's input offset comes from decomposing `row` over
-// the new axes 0..rank-2.
-// IT: index type of the decomposition (32-bit when every index fits: integer division
-// is several times cheaper than in 64 bits, and it runs once per copied unit).  The input
-// strides in g are in units (the host divides them exactly: every stride of an outer axis is
-// a multiple of the row, which is a whole number of units).
-template <typename U, typename IT>
-__global__ void __launch_bounds__(256) k_row_gather(const U *__restrict__ src, U *__restrict__ dst,
-                                                    PermGeom g, int64_t row_units, int64_t total_units) {
-  int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  const IT ru = (IT)row_units;
-  for (; u < total_units; u += step) {
-    const IT uu = (IT)u;
-    IT row = uu / ru;
-    const IT col = uu - row * ru;
-    int64_t off = 0;  // input unit offset of the row start
-    for (int i = g.rank - 2; i >= 0; --i) {
-      const IT d = (IT)g.out_shape[i];
-      const IT q = row / d;
-      off += (int64_t)(row - q * d) * g.in_stride_of_out[i];
-      row = q;
+// ---------------------------------------------------------------- row copy
+// The last new axis equals the last old axis: rows of contiguous elements on both sides, whose
+// order changes.  A CTA writes ROW_THREADS * PER consecutive units (1 to 16 bytes each, whatever
+// divides the rows and the base addresses).  Bound by HBM once the index arithmetic is cheap: the
+// input offset of a row takes a division per outer axis, so it is computed once per row of the
+// chunk, in parallel, into shared memory; a unit then takes one 32-bit division by the row length
+// (a multiply-high by floor(2^32 / d) with one correction) and a look-up, and a thread issues all
+// its loads before the first store.  PER = 1 (small tensors, where one unit's latency is all
+// there is) goes without the table.
+// Measured, a division per axis and unit -> this (read + written TB/s): f64 [2048,4,4,1024]
+// (0,2,1,3) 5.4 -> 6.6, [2047,5,3,1001] 3.0 -> 6.3; f32 [2047,5,3,1001] 1.5 -> 4.0; int16 0.8 ->
+// 2.8, bool 0.4 -> 1.4 (narrow odd rows: bound by the number of element accesses).  Assembling
+// 16-byte outputs from shifted input vectors was faster only for rows above 2 KB of 1- or 4-byte
+// elements and up to 40 % slower for short rows of 8-byte elements.
+constexpr int ROW_THREADS = 256;
+constexpr int row_per(int unit) { return unit >= 16 ? 4 : unit >= 4 ? 8 : 16; }  // units per thread
+
+struct RowGeom {
+  int n;                    // outer axes
+  int64_t ext[kMaxRank];    // their extents, innermost first
+  int64_t ins[kMaxRank];    // input strides (in units)
+  int64_t row;              // units per row
+  uint32_t rec;             // floor(2^32 / row), 2^32 - 1 for one unit per row (rows below 2^31 units)
+  int wide;                 // 64-bit row numbers
+};
+
+// input offset of a row; 32-bit divisions unless the row numbers need more
+__device__ __forceinline__ int64_t row_offset(const RowGeom &g, int64_t row) {
+  int64_t off = 0;
+  if (!g.wide) {
+    uint32_t r = (uint32_t)row;
+    for (int i = 0; i + 1 < g.n; ++i) {
+      const uint32_t d = (uint32_t)g.ext[i], q = r / d;
+      off += (int64_t)(r - q * d) * g.ins[i];
+      r = q;
     }
-    dst[u] = src[off + col];
+    return off + (int64_t)r * g.ins[g.n - 1];
   }
+  for (int i = 0; i + 1 < g.n; ++i) {
+    const int64_t q = row / g.ext[i];
+    off += (row - q * g.ext[i]) * g.ins[i];
+    row = q;
+  }
+  return off + row * g.ins[g.n - 1];
+}
+
+template <typename U, int PER>
+__global__ void __launch_bounds__(ROW_THREADS) k_row_copy(const U *__restrict__ src, U *__restrict__ dst,
+                                                          const __grid_constant__ RowGeom g, int64_t total) {
+  extern __shared__ int64_t row_off[];
+  constexpr int CHUNK = ROW_THREADS * PER;
+  for (int64_t c = (int64_t)blockIdx.x * CHUNK; c < total; c += (int64_t)gridDim.x * CHUNK) {
+    const int64_t r0 = g.wide ? c / g.row : (int64_t)((uint32_t)c / (uint32_t)g.row);  // first row of the chunk
+    const uint32_t c0 = (uint32_t)(c - r0 * g.row);                                 // and the column it starts at
+    const uint32_t cnt = (uint32_t)(total - c < CHUNK ? total - c : CHUNK);
+    const uint32_t len = (uint32_t)g.row;
+    auto split = [&](uint32_t x, uint32_t &col) -> uint32_t {
+      uint32_t q = __umulhi(x, g.rec);
+      if (x - q * len >= len) ++q;  // the estimate is short by at most one
+      col = x - q * len;
+      return q;
+    };
+    if (PER > 1) {
+      uint32_t last;
+      const uint32_t rows = split(c0 + cnt - 1, last) + 1;
+      for (uint32_t i = threadIdx.x; i < rows; i += ROW_THREADS) row_off[i] = row_offset(g, r0 + i);
+      __syncthreads();
+    }
+    U v[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const uint32_t e = threadIdx.x + i * ROW_THREADS;
+      if (e < cnt) {
+        uint32_t col;
+        const uint32_t r = split(c0 + e, col);
+        v[i] = src[(PER > 1 ? row_off[r] : row_offset(g, r0 + r)) + col];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const uint32_t e = threadIdx.x + i * ROW_THREADS;
+      if (e < cnt) dst[c + e] = v[i];
+    }
+    if (PER > 1) __syncthreads();  // the next chunk reuses the table
+  }
+}
+
+template <typename U>
+static void launch_rows(const void *src, void *dst, const RowGeom &g, int64_t total, int nsm, cudaStream_t st) {
+  constexpr int PER = row_per((int)sizeof(U)), CHUNK = ROW_THREADS * PER;
+  if (total < (int64_t)nsm * CHUNK) {
+    k_row_copy<U, 1><<<(unsigned)((total + ROW_THREADS - 1) / ROW_THREADS), ROW_THREADS, 0, st>>>((const U *)src, (U *)dst, g,
+                                                                                             total);
+    return;
+  }
+  const size_t smem = (size_t)(CHUNK / std::max<int64_t>(1, g.row) + 2) * sizeof(int64_t);
+  const int64_t grid = std::min<int64_t>((total + CHUNK - 1) / CHUNK, (int64_t)1 << 30);
+  k_row_copy<U, PER><<<(unsigned)grid, ROW_THREADS, smem, st>>>((const U *)src, (U *)dst, g, total);
 }
 
 // ---------------------------------------------------------------- tiled transpose
@@ -786,13 +849,6 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
   }
   const int nsm = sm_count();
   if (rmap[r - 1] == r - 1) {
-    PermGeom g;
-    g.rank = r;
-    g.n = n;
-    for (int i = 0; i < r; ++i) {
-      g.out_shape[i] = out_shape[i];
-      g.in_stride_of_out[i] = in_stride[rmap[i]];
-    }
     const int64_t L = rshape[r - 1];
     const int64_t bytes_row = L * ES;
     const uintptr_t al = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst);
@@ -802,36 +858,31 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
         vb = cand;
         break;
       }
-    const int64_t scale = vb / ES;  // elements per unit
-    for (int i = 0; i + 1 < r; ++i) g.in_stride_of_out[i] /= scale;  // exact: multiples of L
-    const int64_t row_units = L / scale;
-    const int64_t total_units = n / scale;
-    const int64_t blocks = std::min<int64_t>((total_units + 255) / 256, (int64_t)nsm * 16);
-    const bool small = total_units < (1ll << 31);
-#define CTN_ROW_GATHER(UT)                                                                                        \
-  if (small)                                                                                                     \
-    k_row_gather<UT, uint32_t><<<(unsigned)blocks, 256, 0, st>>>((const UT *)src, (UT *)dst, g, row_units,     \
-                                                                 total_units);                                \
-  else                                                                                                           \
-    k_row_gather<UT, int64_t><<<(unsigned)blocks, 256, 0, st>>>((const UT *)src, (UT *)dst, g, row_units,      \
-                                                                total_units);
-    switch (vb) {
-      case 16:
-        CTN_ROW_GATHER(U128);
-        break;
-      case 8:
-        CTN_ROW_GATHER(uint64_t);
-        break;
-      case 4:
-        CTN_ROW_GATHER(uint32_t);
-        break;
-      case 2:
-        CTN_ROW_GATHER(uint16_t);
-        break;
-      default:
-        CTN_ROW_GATHER(uint8_t);
+    const int64_t unit = vb / ES, row = L / unit, total = n / unit;
+    // rows of 2^31 units and more: one more axis below them (the row is contiguous)
+    RowGeom g;
+    g.n = 0;
+    g.row = row;
+    if (row >= ((int64_t)1 << 31)) {
+      int64_t part = 1 << 30;
+      while (row % part) part >>= 1;
+      g.ext[g.n] = row / part;
+      g.ins[g.n++] = part;
+      g.row = part;
     }
-#undef CTN_ROW_GATHER
+    for (int i = r - 2; i >= 0; --i) {  // innermost outer axis first
+      g.ext[g.n] = out_shape[i];
+      g.ins[g.n++] = in_stride[rmap[i]] / unit;  // exact: multiples of a row
+    }
+    g.rec = g.row > 1 ? (uint32_t)((1ull << 32) / (uint64_t)g.row) : 0xFFFFFFFFu;
+    g.wide = total >= ((int64_t)1 << 32) - 65536;
+    switch (vb) {
+      case 16: launch_rows<U128>(src, dst, g, total, nsm, st); break;
+      case 8: launch_rows<uint64_t>(src, dst, g, total, nsm, st); break;
+      case 4: launch_rows<uint32_t>(src, dst, g, total, nsm, st); break;
+      case 2: launch_rows<uint16_t>(src, dst, g, total, nsm, st); break;
+      default: launch_rows<uint8_t>(src, dst, g, total, nsm, st);
+    }
     CTN_CHECK_LAUNCH();
     return CTN_OK;
   }
