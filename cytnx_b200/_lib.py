@@ -61,6 +61,9 @@ _SIGS = {
     "ctn_dtype_size": (c_size, [c_int]),
     "ctn_permute": (c_int, [c_vp, c_vp, c_int, c_int, P_u64, P_u64, c_vp]),
     "ctn_permute_blocks": (c_int, [c_vp, c_vp, c_int, c_int, c_i64, P_u64, P_i64, P_i64, P_u64, c_vp]),
+    "ctn_permute_plan_create": (c_int, [c_int, c_int, c_i64, P_u64, P_i64, P_i64, P_u64, ctypes.POINTER(c_vp)]),
+    "ctn_permute_plan_run": (c_int, [c_vp, c_vp, c_vp, c_vp]),
+    "ctn_permute_plan_destroy": (None, [c_vp]),
     "ctn_blocks_enumerate": (c_int, [c_int, c_int, P_i32, P_i64, P_i32, P_i64, ctypes.POINTER(c_vp),
                                      P_i64, c_i64, P_i64]),
     "ctn_contract_plan_create": (c_int, [ctypes.POINTER(BlockDesc), ctypes.POINTER(BlockDesc), c_int,

@@ -13,7 +13,7 @@
 // no per-pair kernel launch remain on the device path.  Operand blocks whose
 // legs are already grouped as [noncomm | comm] (or [comm | noncomm]) are read in
 // place (optionally transposed); otherwise all blocks of that operand are permuted
-// once per call into the caller's scratch by the permute kernel.
+// once per call into the caller's scratch, in one launch prepared with the plan.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -24,6 +24,7 @@
 
 #include "ctn_common.h"
 #include "gemm_f64.cuh"
+#include "permute.cuh"
 
 namespace ctn {
 
@@ -111,6 +112,12 @@ struct ctn_contract_plan {
     std::vector<int64_t> src_offs, dst_offs;
     std::vector<uint64_t> mapper;      // new axis i = physical axis mapper[i]
     int64_t elems = 0;                 // elements of the staged copy
+    ctn::BlockPermute *perm = nullptr; // the copy, prepared for execution
+    ~Stage() { ctn::block_permute_destroy(perm); }
+    ctn_status prepare() {
+      return ctn::block_permute_create(CTN_FLOAT64, rank, (int64_t)src_offs.size(), old_shapes.data(), src_offs.data(),
+                                       dst_offs.data(), mapper.data(), &perm);
+    }
   } sl, sr;
   ctn::GroupedGemmF64 gemm;
 };
@@ -178,11 +185,13 @@ extern "C" ctn_status ctn_contract_plan_create(const ctn_block_desc *L, const ct
     std::vector<int64_t> need(nl);
     need.insert(need.end(), cl.begin(), cl.end());
     make_stage(p->sl, *L, need);
+    CTN_TRY(p->sl.prepare());
   }
   if (cls_r == 2) {
     std::vector<int64_t> need(cr);
     need.insert(need.end(), nr.begin(), nr.end());
     make_stage(p->sr, *R, need);
+    CTN_TRY(p->sr.prepare());
   }
 
   // right blocks hashed by their common qindex tuple (BlockUniTensor.cpp:994-1006)
@@ -292,17 +301,13 @@ extern "C" ctn_status ctn_contract_execute(ctn_contract_plan *p, int dtype, cons
   double *sc = (double *)scratch;
   if (p->sl.copy) {
     CTN_REQUIRE(scratch, "ctn_contract_execute: scratch required");
-    CTN_TRY(ctn_permute_blocks(L, sc, CTN_FLOAT64, p->sl.rank, (int64_t)p->sl.src_offs.size(),
-                               p->sl.old_shapes.data(), p->sl.src_offs.data(), p->sl.dst_offs.data(),
-                               p->sl.mapper.data(), stream));
+    CTN_TRY(ctn::block_permute_run(*p->sl.perm, L, sc, st));
     A = sc;
   }
   if (p->sr.copy) {
     CTN_REQUIRE(scratch, "ctn_contract_execute: scratch required");
     double *dst = sc + p->sl.elems;
-    CTN_TRY(ctn_permute_blocks(R, dst, CTN_FLOAT64, p->sr.rank, (int64_t)p->sr.src_offs.size(),
-                               p->sr.old_shapes.data(), p->sr.src_offs.data(), p->sr.dst_offs.data(),
-                               p->sr.mapper.data(), stream));
+    CTN_TRY(ctn::block_permute_run(*p->sr.perm, R, dst, st));
     B = dst;
   }
   return p->gemm.run(A, B, (double *)out, st);

@@ -102,6 +102,34 @@ class _ContractPlan:
             pass
 
 
+class _PermutePlan:
+    """Materialisation of a lazily permuted BlockUniTensor: every block permuted and placed in the
+    Init order of the permuted bonds (which differs from the stored order), prepared once per
+    layout, mapper and dtype."""
+
+    def __init__(self, u: "UniTensor"):
+        self.h = None
+        self.layout = layout_for(u._bonds)
+        self.keep = u._layout  # the cache key holds its id
+        itoi = u._logical_itoi()
+        index = self.layout.index()
+        dst = np.array([self.layout.offs[index[tuple(t)]] for t in itoi.tolist()], dtype=np.int64)
+        shapes = np.ascontiguousarray(u._layout.shapes, dtype=np.uint64)
+        mapper = np.ascontiguousarray(u._mapper, dtype=np.uint64)
+        h = ctypes.c_void_p()
+        _lib.check(_lib.lib().ctn_permute_plan_create(
+            u.dtype(), u.rank(), len(itoi), shapes.ctypes.data_as(_lib.P_u64), u._layout.offs.ctypes.data_as(_lib.P_i64),
+            dst.ctypes.data_as(_lib.P_i64), mapper.ctypes.data_as(_lib.P_u64), ctypes.byref(h)),
+            "BlockUniTensor::contiguous")
+        self.h = h.value
+
+    def __del__(self):
+        try:
+            _lib.lib().ctn_permute_plan_destroy(self.h)
+        except Exception:
+            pass
+
+
 def _desc(lay: BlockLayout, mapper: Optional[Sequence[int]], itoi_logical: np.ndarray,
           shapes_logical: np.ndarray, keep: list) -> BlockDesc:
     rank = itoi_logical.shape[1] if itoi_logical.ndim == 2 else 0
@@ -383,21 +411,14 @@ class UniTensor:
             return UniTensor._new_dense(self._block.contiguous(), self._bonds, self._labels, self._rowrank,
                                         self._name, self._is_diag)
         require_cuda(self._data, "UniTensor::contiguous")
-        lay_new = layout_for(self._bonds)
-        # the logical enumeration order of the permuted bonds differs from the stored
-        # order: materialise every block (permute kernel), then place blocks in the
-        # new Init order.
+        key = ("permute", id(self._layout), tuple(self._mapper), self._data.dtype)
+        plan = _PLANS.get(key)
+        if plan is None:
+            plan = _PLANS[key] = _PermutePlan(self)
+        lay_new = plan.layout
         out = torch.empty(lay_new.nelem, dtype=self._data.dtype, device=self._data.device)
-        itoi_l = self._logical_itoi()
-        idx_new = lay_new.index()
-        dst_offs = np.array([lay_new.offs[idx_new[tuple(t)]] for t in itoi_l.tolist()], dtype=np.int64)
-        old_shapes = np.ascontiguousarray(self._layout.shapes, dtype=np.uint64)
-        mp = np.ascontiguousarray(self._mapper, dtype=np.uint64)
-        _lib.check(_lib.lib().ctn_permute_blocks(
-            self._data.data_ptr(), out.data_ptr(), self.dtype(), self.rank(), len(itoi_l),
-            old_shapes.ctypes.data_as(_lib.P_u64), self._layout.offs.ctypes.data_as(_lib.P_i64),
-            dst_offs.ctypes.data_as(_lib.P_i64), mp.ctypes.data_as(_lib.P_u64), _lib.stream_ptr()),
-            "BlockUniTensor::contiguous")
+        _lib.check(_lib.lib().ctn_permute_plan_run(plan.h, self._data.data_ptr(), out.data_ptr(), _lib.stream_ptr()),
+                   "BlockUniTensor::contiguous")
         return UniTensor._new_block(self._bonds, self._labels, self._rowrank, lay_new, list(range(self.rank())),
                                     out, self._name)
 

@@ -104,6 +104,17 @@ ctn_status ctn_permute_blocks(const void *src, void *dst, int dtype, int rank, i
                               const uint64_t *old_shapes, const int64_t *src_offs,
                               const int64_t *dst_offs, const uint64_t *mapper, void *stream);
 
+/* the same, prepared once for one set of block shapes, offsets and mapper: a run only enqueues
+ * its launches.  A plan holds no device state: any thread, stream and device may run it, also
+ * under stream capture.  No counterpart in the reference (Tensor_impl::contiguous is called per
+ * block, src/BlockUniTensor.cpp:588-708). */
+typedef struct ctn_permute_plan ctn_permute_plan;
+ctn_status ctn_permute_plan_create(int dtype, int rank, int64_t nblocks, const uint64_t *old_shapes,
+                                   const int64_t *src_offs, const int64_t *dst_offs,
+                                   const uint64_t *mapper, ctn_permute_plan **plan);
+ctn_status ctn_permute_plan_run(const ctn_permute_plan *plan, const void *src, void *dst, void *stream);
+void ctn_permute_plan_destroy(ctn_permute_plan *plan);
+
 /* ---------------------------------------------------------------- blocks
  * Enumerate the symmetry-allowed blocks of a tensor with `rank` bonds.
  * sym_types[s]: -1 = U1, 0 = Zn (with modulus sym_n[s]); bond_types[i]: -1 ket, +1 bra;
