@@ -11,8 +11,8 @@
 // tables of one grouped GEMM (gemm_f64.cu): each output block is a task that sums
 // over all of its block pairs, so no per-call hashing, no per-pair allocation, and
 // no per-pair kernel launch remain on the device path.  Operand blocks whose
-// legs are already grouped as [noncomm | comm] (or [comm | noncomm]) are read in
-// place (optionally transposed); otherwise all blocks of that operand are permuted
+// legs (but those of extent 1) are already grouped as [noncomm | comm] (or [comm | noncomm])
+// are read in place (optionally transposed); otherwise all blocks of that operand are permuted
 // once per call into the caller's scratch, in one launch prepared with the plan.
 #include <algorithm>
 #include <cstring>
@@ -124,20 +124,33 @@ struct ctn_contract_plan {
 
 namespace {
 // classify an operand: need logical order `need` (first group then second group)
-// returns 0 = in place (physical == need), 1 = in place transposed (physical ==
-// second ++ first), 2 = needs a permuted copy.
+// returns 0 = in place (every block's memory order is first ++ second), 1 = in place transposed
+// (second ++ first), 2 = needs a permuted copy.  A leg of extent 1 has no place in memory, so each
+// block is judged by its other legs: the MPO and physical legs of a symmetric chain have one
+// state per charge, and without them the environments, wavefunctions and MPO products of a sweep
+// are plain matrices that need no copy, whatever the order of their legs.
 int classify(const ctn_block_desc &d, const std::vector<int64_t> &first, const std::vector<int64_t> &second) {
-  auto phys = [&](int64_t logical) { return d.perm ? d.perm[logical] : logical; };
   bool same = true, swapped = true;
-  int pos = 0;
-  for (int64_t x : first) same &= (phys(x) == pos++);
-  for (int64_t x : second) same &= (phys(x) == pos++);
-  pos = 0;
-  for (int64_t x : second) swapped &= (phys(x) == pos++);
-  for (int64_t x : first) swapped &= (phys(x) == pos++);
-  if (same) return 0;
-  if (swapped) return 1;
-  return 2;
+  for (int64_t b = 0; b < d.nblocks && (same || swapped); ++b) {
+    const int64_t *shape = d.shapes + b * d.rank;
+    int64_t size = 1;
+    for (int i = 0; i < d.rank; ++i) size *= shape[i];
+    if (size == 0) continue;  // nothing to read
+    auto ordered = [&](const std::vector<int64_t> &x, const std::vector<int64_t> &y) {
+      int64_t last = -1;
+      for (const auto *g : {&x, &y})
+        for (int64_t leg : *g) {
+          if (shape[leg] == 1) continue;
+          const int64_t at = d.perm ? d.perm[leg] : leg;
+          if (at < last) return false;
+          last = at;
+        }
+      return true;
+    };
+    same = same && ordered(first, second);
+    swapped = swapped && ordered(second, first);
+  }
+  return same ? 0 : swapped ? 1 : 2;
 }
 
 void make_stage(ctn_contract_plan::Stage &s, const ctn_block_desc &d, const std::vector<int64_t> &need) {
