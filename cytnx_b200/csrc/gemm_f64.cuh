@@ -36,6 +36,12 @@ ctn_status launch_gemm_f64(const double *A, const double *B, double *C, const Ge
                            const GemmPairD *d_pairs, const GemmTileD *d_tiles, int64_t ntiles, int flags,
                            int bm, int bn, cudaStream_t st);
 
+// the element runs of k_scaled_sum (vectors of m elements when col, else of n)
+void build_chunks_f64(const std::vector<GemmTaskD> &tasks, bool col, std::vector<GemmTileD> &tiles);
+ctn_status launch_scaled_sum_f64(const double *A, const double *B, double *C, const GemmTaskD *d_tasks,
+                                 const GemmPairD *d_pairs, const GemmTileD *d_tiles, int64_t ntiles, bool col,
+                                 cudaStream_t st);
+
 // Host tables + their device copy (uploaded once, on the first launch on a device).
 struct GroupedGemmF64 {
   std::vector<GemmTaskD> tasks;
@@ -47,6 +53,20 @@ struct GroupedGemmF64 {
   int flags = 0;          // operand orientation shared by every pair of the plan
   int bm = 64, bn = 64;   // tile: 64 x 64; 64 x 32 when 64 x 64 would not fill the SMs; 32 x 32 for small blocks
   bool mixed = false;     // pairs disagree on the orientation (rejected at run time)
+  int scaled = 0;         // 1: every product is a column vector times a scalar, 2: a row vector, 0: GEMM
+
+  // whether all products are scalar times a contiguous vector (k_scaled_sum)
+  bool scaled_sum(bool col) const {
+    for (const auto &t : tasks) {
+      if (col ? t.n != 1 || t.ldc != 1 : t.m != 1) return false;
+      for (int p = 0; p < t.pair_count; ++p) {
+        const GemmPairD &pr = pairs[t.pair_begin + p];
+        if (pr.k > 1) return false;
+        if (col ? !(pr.flags & 1) && pr.lda != 1 : (pr.flags & 2) && pr.ldb != 1) return false;
+      }
+    }
+    return !tasks.empty();
+  }
 
   // products the tiles execute, with K padded to the 16-deep stages
   double executed(int tm, int tn) const {
@@ -65,10 +85,12 @@ struct GroupedGemmF64 {
     // tiles (D ~ 1000 two-site problems: sectors of 2-68 states): 32 x 32 tiles
     bm = 64;
     bn = 64;
-    build_tiles_f64(tasks, pairs, tiles, bm, bn);
-    if (tiles.size() < F64_NARROW_BELOW * 148) bn = 32;
-    if (executed(bm, bn) > F64_SMALL_PADDING * executed(32, 32)) bm = bn = 32;
-    if (bm != 64 || bn != 64) build_tiles_f64(tasks, pairs, tiles, bm, bn);
+    scaled = scaled_sum(true) ? 1 : scaled_sum(false) ? 2 : 0;
+    if (scaled) build_chunks_f64(tasks, scaled == 1, tiles);
+    else build_tiles_f64(tasks, pairs, tiles, bm, bn);
+    if (!scaled && tiles.size() < F64_NARROW_BELOW * 148) bn = 32;
+    if (!scaled && executed(bm, bn) > F64_SMALL_PADDING * executed(32, 32)) bm = bn = 32;
+    if (!scaled && (bm != 64 || bn != 64)) build_tiles_f64(tasks, pairs, tiles, bm, bn);
     flags = pairs.empty() ? 0 : (pairs[0].flags & 3);
     mixed = false;
     for (const auto &p : pairs) mixed |= ((p.flags & 3) != flags);
@@ -111,6 +133,7 @@ struct GroupedGemmF64 {
     const GemmTaskD *dt = (const GemmTaskD *)p;
     const GemmPairD *dp = (const GemmPairD *)(p + tasks.size() * sizeof(GemmTaskD));
     const GemmTileD *dl = (const GemmTileD *)(p + tasks.size() * sizeof(GemmTaskD) + pairs.size() * sizeof(GemmPairD));
+    if (scaled) return launch_scaled_sum_f64(A, B, C, dt, dp, dl, (int64_t)tiles.size(), scaled == 1, st);
     return launch_gemm_f64(A, B, C, dt, dp, dl, (int64_t)tiles.size(), flags, bm, bn, st);
   }
   ~GroupedGemmF64() {
