@@ -6,7 +6,7 @@
 // src/BlockUniTensor.cpp:1180-1223) or one Gemm_Batch group entry (MKL build,
 // :1114-1177) per block pair; the reference's GPU Gemm_Batch is a serial loop of
 // cublasDgemm calls (src/backend/linalg_internal_gpu/cuGemm_Batch_internal.cu:23-64).
-// Here a CTA owns one 64x64 tile of one output block and walks the whole K range of
+// Here a CTA owns one 64x32 or 32x32 tile of one output block and walks the whole K range of
 // all its pairs, so every output element is written exactly once (no atomics, no
 // zero-fill pass; tasks with no pair write zeros, matching Init's zeros blocks).
 // Operands are read in place from the block storage with per-pair leading
@@ -22,14 +22,17 @@
 namespace ctn {
 
 namespace {
-constexpr int BK = 16;  // k depth of a stage; tiles are BM x BN = 64 x 64, 64 x 32 or 32 x 32
+constexpr int BK = 16;  // k depth of a stage; tiles are BM x BN = 64 x 32 or 32 x 32
 constexpr int PAD = 4;
 constexpr int NTHREADS = 128;
 
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool pred) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  int sz = pred ? 8 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
+// 8 bytes global -> shared (a shared-window address); cp_async8_zfill copies nothing and writes
+// zeros when `bytes` is 0
+__device__ __forceinline__ void cp_async8(uint32_t smem, const void *gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async8_zfill(uint32_t smem, const void *gmem, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem), "l"(gmem), "r"(bytes));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -58,48 +61,57 @@ struct SmemT {
   double B[2][TB ? BN : BK][(TB ? BK : BN) + PAD];
 };
 
-template <bool TA, bool TB, int BM, int BN>
-__device__ __forceinline__ void load_stage(SmemT<TA, TB, BM, BN> &sm, int buf, const double *__restrict__ A,
-                                           const double *__restrict__ B, const GemmPairD &p, int m, int n,
-                                           int m0, int n0, int k0) {
-  const int tid = threadIdx.x;
-  const double *Ap = A + p.a_off;
-  const double *Bp = B + p.b_off;
-#pragma unroll
-  for (int i = 0; i < (BM * BK) / NTHREADS; ++i) {
-    const int idx = tid + i * NTHREADS;
-    if (!TA) {  // A[m][k]: k contiguous
-      const int mm = idx / BK, kk = idx % BK;
-      const int gm = m0 + mm, gk = k0 + kk;
-      const bool ok = gm < m && gk < p.k;
-      cp_async8(&sm.A[buf][mm][kk], ok ? Ap + (int64_t)gm * p.lda + gk : Ap, ok);
-    } else {  // A stored [k][m]: m contiguous
-      const int kk = idx / BM, mm = idx % BM;
-      const int gm = m0 + mm, gk = k0 + kk;
-      const bool ok = gm < m && gk < p.k;
-      cp_async8(&sm.A[buf][kk][mm], ok ? Ap + (int64_t)gk * p.lda + gm : Ap, ok);
-    }
+// One operand's side of the load cursor: this thread's share of the W x BK slices of the current
+// pair.  KC: k is the contiguous axis of the source (and of the stage), else the rows are.  All that
+// does not change from slice to slice is set up once per pair, so that an element costs its copy
+// and one 64-bit add: the loads' index arithmetic (20 instructions an element) was three quarters
+// of the instructions of the main loop and kept the DMMA pipe at 76 %.
+template <bool KC, int W, int PITCH>
+struct SliceCursor {
+  static constexpr int LINE = KC ? BK : W;          // contiguous elements of a line of the stage
+  static constexpr int LPP = NTHREADS / LINE;       // lines copied per pass
+  static constexpr int PASSES = (KC ? W : BK) / LPP;
+  static constexpr uint32_t DST = LPP * PITCH * 8;  // bytes between passes in the stage
+  const double *p;  // this thread's element of pass 0 of the next slice
+  int64_t step;     // elements between passes
+  int64_t adv;      // elements between slices
+  __device__ __forceinline__ static int line() { return threadIdx.x / LINE; }
+  __device__ __forceinline__ static int pos() { return threadIdx.x % LINE; }
+  __device__ __forceinline__ static uint32_t offset() { return (uint32_t)(line() * PITCH + pos()) * 8; }
+  __device__ __forceinline__ void start(const double *src, int ld, int r0) {
+    p = KC ? src + (int64_t)(r0 + line()) * ld + pos() : src + (int64_t)line() * ld + r0 + pos();
+    step = LPP * (int64_t)ld;
+    adv = KC ? BK : BK * (int64_t)ld;
   }
+  // whole slice: all W rows and BK k inside the block
+  __device__ __forceinline__ void load(uint32_t dst) {
+    const double *q = p;
 #pragma unroll
-  for (int i = 0; i < (BN * BK) / NTHREADS; ++i) {
-    const int idx = tid + i * NTHREADS;
-    if (!TB) {  // B[k][n]: n contiguous
-      const int kk = idx / BN, nn = idx % BN;
-      const int gn = n0 + nn, gk = k0 + kk;
-      const bool ok = gn < n && gk < p.k;
-      cp_async8(&sm.B[buf][kk][nn], ok ? Bp + (int64_t)gk * p.ldb + gn : Bp, ok);
-    } else {  // B stored [n][k]: k contiguous
-      const int nn = idx / BK, kk = idx % BK;
-      const int gn = n0 + nn, gk = k0 + kk;
-      const bool ok = gn < n && gk < p.k;
-      cp_async8(&sm.B[buf][nn][kk], ok ? Bp + (int64_t)gn * p.ldb + gk : Bp, ok);
-    }
+    for (int i = 0; i < PASSES; ++i, q += step) cp_async8(dst + i * DST, q);
+    p += adv;
   }
-}
+  // `rows` rows and `k` k left in the block: rows past it are not loaded (they only reach output
+  // rows that are not stored), k past it is zero-filled (from `any`, which is not read)
+  __device__ __forceinline__ void load_edge(uint32_t dst, int rows, int k, const double *any) {
+    const double *q = p;
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i, q += step) {
+      const int l = line() + i * LPP, x = pos();
+      const bool ok = (KC ? x : l) < k;
+      if ((KC ? l : x) < rows) cp_async8_zfill(dst + i * DST, ok ? q : any, ok ? 8 : 0);
+    }
+    p += adv;
+  }
+};
 
-// Each of the 4 warps computes a (BM / 2) x (BN / 2) quarter of the tile: 64 x 64 tiles 2 x 4
-// m16n8 products per k step, 64 x 32 tiles 2 x 2 (plans with too few 64 x 64 tiles to fill the
-// SMs), 32 x 32 tiles 1 x 2 (plans of small blocks, where 64-row tiles are mostly padding).
+// Each of the 4 warps computes a (BM / 2) x (BN / 2) quarter of the tile: 64 x 32 tiles 2 x 2
+// m16n8 products per k step, 32 x 32 tiles (plans of small blocks, where 64 rows are mostly
+// padding) 1 x 2.  Bound by the DMMA pipe, which runs at 128 cycles a product and SM quarter, and by
+// how well the other warps' instructions hide behind it.  Two-site FP64 matvec, with the loads'
+// arithmetic inside the stage and 64 x 64 tiles -> this: D=4096 635 -> 555 us, D=3000 283 -> 249,
+// D=2048 126 -> 105, D=1500 61 -> 52, D=1024 33.0 -> 31.8.  Warps with tiles and stages of their own, which
+// skip the padding (1.11 instead of 1.36 times the useful products at D=4096), were slower (637 us
+// and more: ten warps per SM do not hide their own load instructions).
 template <bool TA, bool TB, int BM, int BN>
 __global__ void __launch_bounds__(NTHREADS) k_gemm_grouped_f64(
     const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C,
@@ -108,13 +120,19 @@ __global__ void __launch_bounds__(NTHREADS) k_gemm_grouped_f64(
   constexpr int MI = BM / 32;  // m16 products per warp
   constexpr int NJ = BN / 16;  // n8 products per warp
   __shared__ __align__(16) SmemT<TA, TB, BM, BN> sm;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = (warp >> 1) * (BM / 2), wn = (warp & 1) * (BN / 2);
+  using CA = SliceCursor<!TA, BM, (TA ? BM : BK) + PAD>;
+  using CB = SliceCursor<TB, BN, (TB ? BK : BN) + PAD>;
+  const uint32_t da0 = (uint32_t)__cvta_generic_to_shared(&sm.A[0][0][0]) + CA::offset();
+  const uint32_t db0 = (uint32_t)__cvta_generic_to_shared(&sm.B[0][0][0]) + CB::offset();
+  const int lane = threadIdx.x & 31;
   const int g = lane >> 2, t4 = lane & 3;
   for (int64_t ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
     const GemmTileD tile = tiles[ti];
     const GemmTaskD task = tasks[tile.task];
     const int m0 = tile.m0, n0 = tile.n0;
+    const int mr = task.m - m0, nr = task.n - n0;  // rows and columns of the block from here on
+    const int quarter = threadIdx.x >> 5;
+    const int wm = (quarter >> 1) * (BM / 2), wn = (quarter & 1) * (BN / 2);
     double acc[MI][NJ][4];
 #pragma unroll
     for (int i = 0; i < MI; ++i)
@@ -123,30 +141,53 @@ __global__ void __launch_bounds__(NTHREADS) k_gemm_grouped_f64(
 #pragma unroll
         for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0;
 
-    // flattened (pair, k-tile) iteration with a 2-deep cp.async pipeline
-    int pi = 0, kt = 0;
-    const int npairs = task.pair_count;
-    while (pi < npairs && pairs[task.pair_begin + pi].k <= 0) ++pi;
-    int buf = 0;
-    bool have = pi < npairs;
-    GemmPairD cur;
-    if (have) {
-      cur = pairs[task.pair_begin + pi];
-      load_stage<TA, TB, BM, BN>(sm, 0, A, B, cur, task.m, task.n, m0, n0, 0);
-    }
-    cp_async_commit();
-    while (have) {
-      int npi = pi, nkt = kt + 1;
-      GemmPairD nxt = cur;
-      if (nkt * BK >= cur.k) {
-        nkt = 0;
-        ++npi;
-        while (npi < npairs && pairs[task.pair_begin + npi].k <= 0) ++npi;
-        if (npi < npairs) nxt = pairs[task.pair_begin + npi];
+    // flattened (pair, k) iteration with a 2-deep cp.async pipeline; the next pair's descriptor is
+    // fetched when a pair begins
+    const GemmPairD *next = pairs + task.pair_begin, *const last = next + task.pair_count;
+    GemmPairD np;
+    int kleft = 0;
+    CA ca;
+    CB cb;
+    auto fetch = [&] {  // the next pair with work
+      np.k = 0;
+      while (next < last) {
+        np = *next++;
+        if (np.k > 0) break;
       }
-      const bool have_next = npi < npairs;
-      if (have_next) load_stage<TA, TB, BM, BN>(sm, buf ^ 1, A, B, nxt, task.m, task.n, m0, n0, nkt * BK);
+    };
+    auto begin_pair = [&] {
+      kleft = np.k > 0 ? np.k : 0;
+      if (kleft) {
+        ca.start(A + np.a_off, np.lda, m0);
+        cb.start(B + np.b_off, np.ldb, n0);
+        fetch();
+      }
+    };
+    fetch();
+    begin_pair();
+    const bool rows_whole = mr >= BM && nr >= BN;
+    auto issue = [&](int slot) -> bool {
+      const bool have = kleft > 0;
+      if (have) {
+        const uint32_t da = da0 + (uint32_t)slot * (uint32_t)sizeof(sm.A[0]);
+        const uint32_t db = db0 + (uint32_t)slot * (uint32_t)sizeof(sm.B[0]);
+        if (rows_whole && kleft >= BK) {
+          ca.load(da);
+          cb.load(db);
+        } else {
+          ca.load_edge(da, mr, kleft, A);
+          cb.load_edge(db, nr, kleft, B);
+        }
+        kleft -= BK;
+        if (kleft <= 0) begin_pair();
+      }
       cp_async_commit();
+      return have;
+    };
+    int buf = 0;
+    bool have = issue(0);
+    while (have) {
+      const bool have_next = issue(buf ^ 1);
       cp_async_wait<1>();
       __syncthreads();
       double a[MI][8], b[NJ][4];
@@ -170,9 +211,6 @@ __global__ void __launch_bounds__(NTHREADS) k_gemm_grouped_f64(
         for (int j = 0; j < NJ; ++j) dmma_16x8x16(acc[i][j], a[i], b[j]);
       __syncthreads();
       buf ^= 1;
-      pi = npi;
-      kt = nkt;
-      cur = nxt;
       have = have_next;
     }
     cp_async_wait<0>();
@@ -274,40 +312,36 @@ ctn_status launch_scaled_sum_f64(const double *A, const double *B, double *C, co
   return CTN_OK;
 }
 
+namespace {
+template <bool TA, bool TB, int BM, int BN>
+ctn_status launch_gemm(const double *A, const double *B, double *C, const GemmTaskD *d_tasks, const GemmPairD *d_pairs,
+                       const GemmTileD *d_tiles, int64_t ntiles, int nsm, cudaStream_t st) {
+  const int64_t grid = std::min<int64_t>(ntiles, (int64_t)nsm * 12);
+  k_gemm_grouped_f64<TA, TB, BM, BN><<<(unsigned)grid, NTHREADS, 0, st>>>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles);
+  CTN_CHECK_LAUNCH();
+  return CTN_OK;
+}
+template <bool TA, bool TB>
+ctn_status launch_tiles(const double *A, const double *B, double *C, const GemmTaskD *d_tasks, const GemmPairD *d_pairs,
+                        const GemmTileD *d_tiles, int64_t ntiles, int bm, int nsm, cudaStream_t st) {
+  if (bm == 32) return launch_gemm<TA, TB, 32, 32>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, nsm, st);
+  return launch_gemm<TA, TB, 64, 32>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, nsm, st);
+}
+}  // namespace
+
 ctn_status launch_gemm_f64(const double *A, const double *B, double *C, const GemmTaskD *d_tasks,
                            const GemmPairD *d_pairs, const GemmTileD *d_tiles, int64_t ntiles, int flags,
-                           int bm, int bn, cudaStream_t st) {
+                           int bm, cudaStream_t st) {
   if (ntiles == 0) return CTN_OK;
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  // 128 threads, ~17 KB smem: up to 8+ CTAs per SM resident
-  const int64_t grid = std::min<int64_t>(ntiles, (int64_t)nsm * 12);
-  auto go = [&](auto kern) { kern<<<(unsigned)grid, NTHREADS, 0, st>>>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles); };
-  if (bm == 32) {
-    switch (flags & 3) {
-      case 0: go(k_gemm_grouped_f64<false, false, 32, 32>); break;
-      case 1: go(k_gemm_grouped_f64<true, false, 32, 32>); break;
-      case 2: go(k_gemm_grouped_f64<false, true, 32, 32>); break;
-      default: go(k_gemm_grouped_f64<true, true, 32, 32>); break;
-    }
-  } else if (bn == 32) {
-    switch (flags & 3) {
-      case 0: go(k_gemm_grouped_f64<false, false, 64, 32>); break;
-      case 1: go(k_gemm_grouped_f64<true, false, 64, 32>); break;
-      case 2: go(k_gemm_grouped_f64<false, true, 64, 32>); break;
-      default: go(k_gemm_grouped_f64<true, true, 64, 32>); break;
-    }
-  } else {
-    switch (flags & 3) {
-      case 0: go(k_gemm_grouped_f64<false, false, 64, 64>); break;
-      case 1: go(k_gemm_grouped_f64<true, false, 64, 64>); break;
-      case 2: go(k_gemm_grouped_f64<false, true, 64, 64>); break;
-      default: go(k_gemm_grouped_f64<true, true, 64, 64>); break;
-    }
+  switch (flags & 3) {
+    case 0: return launch_tiles<false, false>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, nsm, st);
+    case 1: return launch_tiles<true, false>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, nsm, st);
+    case 2: return launch_tiles<false, true>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, nsm, st);
+    default: return launch_tiles<true, true>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, nsm, st);
   }
-  CTN_CHECK_LAUNCH();
-  return CTN_OK;
 }
 
 }  // namespace ctn

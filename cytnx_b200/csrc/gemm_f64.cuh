@@ -8,12 +8,10 @@
 
 namespace ctn {
 
-#ifndef F64_NARROW_BELOW
-#define F64_NARROW_BELOW 6  // 64 x 32 tiles when a plan has fewer 64 x 64 tiles than this many per SM
-#endif
-#ifndef F64_SMALL_PADDING
-#define F64_SMALL_PADDING 1.25  // 32 x 32 tiles when the wider tiles execute this many times the products of 32 x 32 tiles
-#endif
+// 32 x 32 tiles when 64 x 32 tiles execute more than this many times their products: blocks of up
+// to a few hundred rows (D=2048 two-site matvec 105 us against 113), the wider tiles where their
+// padding is small (D=4096: 555 us against 567).  64 x 64 tiles were slower throughout (580 us).
+constexpr double F64_NARROW_PADDING = 1.12;
 
 struct GemmTaskD {
   int64_t c_off;
@@ -34,7 +32,7 @@ void build_tiles_f64(const std::vector<GemmTaskD> &tasks, const std::vector<Gemm
                      std::vector<GemmTileD> &tiles, int bm, int bn);
 ctn_status launch_gemm_f64(const double *A, const double *B, double *C, const GemmTaskD *d_tasks,
                            const GemmPairD *d_pairs, const GemmTileD *d_tiles, int64_t ntiles, int flags,
-                           int bm, int bn, cudaStream_t st);
+                           int bm, cudaStream_t st);
 
 // the element runs of k_scaled_sum (vectors of m elements when col, else of n)
 void build_chunks_f64(const std::vector<GemmTaskD> &tasks, bool col, std::vector<GemmTileD> &tiles);
@@ -51,7 +49,7 @@ struct GroupedGemmF64 {
   int d_dev = -1;
   double flops = 0.0;
   int flags = 0;          // operand orientation shared by every pair of the plan
-  int bm = 64, bn = 64;   // tile: 64 x 64; 64 x 32 when 64 x 64 would not fill the SMs; 32 x 32 for small blocks
+  int bm = 64;            // rows of a tile of 32 columns
   bool mixed = false;     // pairs disagree on the orientation (rejected at run time)
   int scaled = 0;         // 1: every product is a column vector times a scalar, 2: a row vector, 0: GEMM
 
@@ -79,18 +77,13 @@ struct GroupedGemmF64 {
     return w;
   }
   void finalize() {
-    // fewer than six 64 x 64 tiles per SM (148 SMs; about 1.5 waves of four resident CTAs):
-    // 64 x 32 tiles, twice as many CTAs, less padding on narrow groups and a fuller last wave;
-    // blocks so small that these tiles execute F64_SMALL_PADDING times the products of 32 x 32
-    // tiles (D ~ 1000 two-site problems: sectors of 2-68 states): 32 x 32 tiles
-    bm = 64;
-    bn = 64;
     scaled = scaled_sum(true) ? 1 : scaled_sum(false) ? 2 : 0;
-    if (scaled) build_chunks_f64(tasks, scaled == 1, tiles);
-    else build_tiles_f64(tasks, pairs, tiles, bm, bn);
-    if (!scaled && tiles.size() < F64_NARROW_BELOW * 148) bn = 32;
-    if (!scaled && executed(bm, bn) > F64_SMALL_PADDING * executed(32, 32)) bm = bn = 32;
-    if (!scaled && (bm != 64 || bn != 64)) build_tiles_f64(tasks, pairs, tiles, bm, bn);
+    if (scaled) {
+      build_chunks_f64(tasks, scaled == 1, tiles);
+    } else {
+      bm = executed(64, 32) > F64_NARROW_PADDING * executed(32, 32) ? 32 : 64;
+      build_tiles_f64(tasks, pairs, tiles, bm, 32);
+    }
     flags = pairs.empty() ? 0 : (pairs[0].flags & 3);
     mixed = false;
     for (const auto &p : pairs) mixed |= ((p.flags & 3) != flags);
@@ -134,7 +127,7 @@ struct GroupedGemmF64 {
     const GemmPairD *dp = (const GemmPairD *)(p + tasks.size() * sizeof(GemmTaskD));
     const GemmTileD *dl = (const GemmTileD *)(p + tasks.size() * sizeof(GemmTaskD) + pairs.size() * sizeof(GemmPairD));
     if (scaled) return launch_scaled_sum_f64(A, B, C, dt, dp, dl, (int64_t)tiles.size(), scaled == 1, st);
-    return launch_gemm_f64(A, B, C, dt, dp, dl, (int64_t)tiles.size(), flags, bm, bn, st);
+    return launch_gemm_f64(A, B, C, dt, dp, dl, (int64_t)tiles.size(), flags, bm, st);
   }
   ~GroupedGemmF64() {
     if (d_mem) cudaFree(d_mem);
