@@ -42,6 +42,17 @@ ctn_status krylov_step_f64(const double *w, const double *u, const double *up, c
 ctn_status krylov_step_f64(const float *w, const double *u, const double *up, const double *q, double *dst,
                            int64_t n, const double *s, const double *sp, double *out_alpha, double *out_gamma,
                            double *nrm, double *ws, double *ws2, unsigned *err, cudaStream_t st);
+// one step of the plain recurrence in one cooperative launch: *out_alpha = <w, p1>, v = w - alpha p1 -
+// *beta p0 (p0 may be null), *out_beta = |v|, dst = v / |v|; ws: the reduction workspace (zeroed
+// before its first use).  A barrier wait that runs out sets *err (device word, zeroed by the
+// caller) and alpha and beta to NaN.  CTN_ERR_UNSUPPORTED without launching when the device has
+// no cooperative launch.
+ctn_status lanczos_gnd_step_f64(const double *w, const double *p1, const double *p0, double *dst, int64_t n,
+                                const double *beta, double *out_alpha, double *out_beta, double *ws, unsigned *err,
+                                cudaStream_t st);
+ctn_status lanczos_gnd_step_f64(const float *w, const double *p1, const double *p0, double *dst, int64_t n,
+                                const double *beta, double *out_alpha, double *out_beta, double *ws, unsigned *err,
+                                cudaStream_t st);
 ctn_status div_copy_f64(const double *x, double *y, int64_t n, const double *a, cudaStream_t st);
 ctn_status combine_f64(const double *K, int64_t n, int m, const double *c, double *out, cudaStream_t st);
 // block Krylov helpers (basis V: m vectors of n doubles back to back)

@@ -186,8 +186,8 @@ static ctn_status pinned_scalars(double **out) {
 // re-solved each iteration, stop on |dE| < cvgcrit or beta == 0; the Ritz vector is
 // the combination of the stored Krylov vectors.  The vectors stay on the device; the
 // two scalars per iteration come to the host as the reference's .item() calls do.
-// speculate: queue iteration i+1 on the device before the host solves iteration i's
-// tridiagonal, so the host solve runs under the next matvec; the iteration queued after the
+// speculate: queue iteration i+1 on the device before iteration i has finished, so neither its
+// launches nor the host's tridiagonal solve hold the device up; the iteration queued after the
 // last one runs and is discarded (one extra matvec, results unchanged).  Only for matvecs
 // without side effects.
 ctn_status lanczos_gnd(int (*mv)(void *, const double *, double *, void *), void *user, const double *psi0,
@@ -199,7 +199,8 @@ ctn_status lanczos_gnd(int (*mv)(void *, const double *, double *, void *), void
   double *w = work;                      // new_psi
   // device scalars: [0] |psi0|, [1] alpha, [2] / [3] the norms of w, alternately written by one
   // update and read as beta (the coefficient of psi_{i-1}) by the next, so no value travels
-  // back to the device; one host read of [1..3] per iteration (the reference's .item() calls)
+  // back to the device, [4] error word of the fused step; one host read of [1..4] per iteration
+  // (the reference's .item() calls)
   double *scal = work + n;
   double *ws = work + n + 8;             // reduction workspace (zeroed below)
   double *cdev = ws + reduce_ws_bytes() / sizeof(double);
@@ -215,31 +216,42 @@ ctn_status lanczos_gnd(int (*mv)(void *, const double *, double *, void *), void
   } guard{ev};
   for (int k = 0; k < 2; ++k) CTN_CUDA(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
   CTN_CUDA(cudaMemsetAsync(ws, 0, reduce_ws_bytes(), st));
+  CTN_CUDA(cudaMemsetAsync(scal, 0, 8 * sizeof(double), st));
+  unsigned *err = reinterpret_cast<unsigned *>(scal + 4);
+  bool fused = true;  // the step after the matvec is one cooperative launch while the device supports it
   // psi_1 = Tin / |Tin|
   CTN_TRY(nrm2_f64(psi0, n, scal + 0, ws, st));
   CTN_CUDA(cudaMemcpyAsync(pin + 8, scal + 0, sizeof(double), cudaMemcpyDeviceToHost, st));
   CTN_CUDA(cudaStreamSynchronize(st));
   CTN_REQUIRE(pin[8] > 0 && std::isfinite(pin[8]), "[Lanczos] initial vector has zero or non-finite norm");
   CTN_TRY(div_copy_f64(psi0, krylov, n, scal + 0, st));
-  // iteration i on the device: (i >= 1) psi_i = w / beta_{i-1}; w = H psi_i; alpha_i = <w, psi_i>;
-  // w -= alpha_i psi_i + beta_{i-1} psi_{i-1}; beta_i = |w|; alpha_i, beta_i -> pinned slot i & 1
-  // w_f32 (split-precision matvecs): mv writes w as n floats, the update writes its FP64 result
-  // straight into the next Krylov slot, which the next iteration scales in place
+  // iteration i on the device: w = H psi_i; alpha_i = <w, psi_i>; w -= alpha_i psi_i + beta_{i-1}
+  // psi_{i-1}; beta_i = |w|; psi_{i+1} = w / beta_i; alpha_i, beta_i -> pinned slot i & 1.  The three
+  // vector operations are one launch, or three kernels of which the last is left to the next iteration.
+  // w_f32 (split-precision matvecs): mv writes w as n floats; the three-kernel form's update writes its
+  // FP64 result straight into the next Krylov slot, which the next iteration scales in place
   auto queue = [&](int i) -> ctn_status {
     double *pi = krylov + (int64_t)i * n;
+    const double *po = i ? pi - n : nullptr;
     double *b_new = scal + 2 + (i & 1);
     const double *b_old = i ? scal + 2 + ((i - 1) & 1) : nullptr;
-    if (i) CTN_TRY(div_copy_f64(w_f32 ? pi : w, pi, n, b_old, st));
+    if (i && !fused) CTN_TRY(div_copy_f64(w_f32 ? pi : w, pi, n, b_old, st));
     if (mv(user, pi, w, st) != 0) return CTN_ERR_CUDA;
-    if (w_f32) {
-      const float *wf = reinterpret_cast<const float *>(w);
-      CTN_TRY(dot_f64(wf, pi, n, scal + 1, ws, st));
-      CTN_TRY(lanczos_update_to_f64(wf, pi, i ? pi - n : nullptr, pi + n, n, scal + 1, b_old, b_new, ws, st));
-    } else {
-      CTN_TRY(dot_f64(w, pi, n, scal + 1, ws, st));
-      CTN_TRY(lanczos_update_f64(w, pi, i ? pi - n : nullptr, n, scal + 1, b_old, b_new, ws, st));
+    const float *wf = reinterpret_cast<const float *>(w);
+    if (fused) {
+      const ctn_status r = w_f32 ? lanczos_gnd_step_f64(wf, pi, po, pi + n, n, b_old, scal + 1, b_new, ws, err, st)
+                                 : lanczos_gnd_step_f64(w, pi, po, pi + n, n, b_old, scal + 1, b_new, ws, err, st);
+      if (r == CTN_ERR_UNSUPPORTED) fused = false;  // found in iteration 0, nothing launched
+      else CTN_TRY(r);
     }
-    CTN_CUDA(cudaMemcpyAsync(pin + 4 * (i & 1), scal + 1, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (!fused && w_f32) {
+      CTN_TRY(dot_f64(wf, pi, n, scal + 1, ws, st));
+      CTN_TRY(lanczos_update_to_f64(wf, pi, po, pi + n, n, scal + 1, b_old, b_new, ws, st));
+    } else if (!fused) {
+      CTN_TRY(dot_f64(w, pi, n, scal + 1, ws, st));
+      CTN_TRY(lanczos_update_f64(w, pi, po, n, scal + 1, b_old, b_new, ws, st));
+    }
+    CTN_CUDA(cudaMemcpyAsync(pin + 4 * (i & 1), scal + 1, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
     CTN_CUDA(cudaEventRecord(ev[i & 1], st));
     return CTN_OK;
   };
@@ -249,11 +261,17 @@ ctn_status lanczos_gnd(int (*mv)(void *, const double *, double *, void *), void
   CTN_TRY(queue(0));
   for (int i = 0; i < maxiter; ++i) {
     it = i + 1;
+    // nothing of the next iteration depends on the host, so it is queued before this one has
+    // finished: the device does not wait for the launches (a breakdown leaves it zeros to work on)
+    if (speculate && i + 1 < maxiter) CTN_TRY(queue(i + 1));
     CTN_CUDA(cudaEventSynchronize(ev[i & 1]));
     const double alpha = pin[4 * (i & 1)], beta = pin[4 * (i & 1) + 1 + (i & 1)];
+    if (pin[4 * (i & 1) + 3] != 0.0) {
+      set_error("[Lanczos] the grid barrier of a fused step gave up waiting");
+      return CTN_ERR_TIMEOUT;
+    }
     As.push_back(alpha);
     const bool more = beta != 0.0 && i + 1 < maxiter;
-    if (speculate && more) CTN_TRY(queue(i + 1));
     const int m = (int)As.size();
     evals.assign(m, 0.0);
     // eigenvalues only inside the loop: the Ritz vector is needed once, after it
