@@ -157,5 +157,7 @@ def stream_ptr(stream=None) -> int:
     """Raw cudaStream_t of a torch stream (default: the current stream)."""
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return int(s.cuda_stream)
+    if stream is not None:
+        return int(stream.cuda_stream)
+    # the raw handle without building a torch.cuda.Stream (5 us of a 15 us call)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())

@@ -73,7 +73,6 @@ def redirect_all(u: UniTensor) -> UniTensor:
     and its layout are shared."""
     v = u.clone_meta()
     v._bonds = [b.redirect() for b in u._bonds]
-    v._is_braket = v._update_braket()
     return v
 
 

@@ -9,6 +9,8 @@ data movement on a CUDA tensor runs the library's own kernels through the C ABI.
 from __future__ import annotations
 
 import ctypes
+import functools
+import math
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -42,11 +44,13 @@ class _Type:
     def to_torch(self, dt: int) -> torch.dtype:
         return self._torch[dt]
 
+    _ids = {v: k for k, v in _torch.items()}
+
     def from_torch(self, dt: torch.dtype) -> int:
-        for k, v in self._torch.items():
-            if v == dt:
-                return k
-        raise CytnxError(f"unsupported dtype {dt}")
+        k = self._ids.get(dt)
+        if k is None:
+            raise CytnxError(f"unsupported dtype {dt}")
+        return k
 
     def getname(self, dt: int) -> str:
         return self._names.get(dt, "Void")
@@ -84,7 +88,7 @@ Device = _Device()
 
 
 def require_cuda(t: torch.Tensor, what: str) -> None:
-    if t.device.type != "cuda":
+    if not t.is_cuda:
         raise CytnxError(f"[{what}] cytnx_b200 computes on CUDA devices only; "
                          f"move the tensor to a GPU with .to(cytnx_b200.Device.cuda)")
 
@@ -134,8 +138,24 @@ class _BondType:
 bondType = _BondType()
 
 
+class _Value:
+    """A tuple compared by value whose hash is taken once (the keys of layouts and plans)."""
+
+    __slots__ = ("_v", "_h")
+
+    def __init__(self, v: tuple):
+        self._v, self._h = v, hash(v)
+
+    def __hash__(self) -> int:
+        return self._h
+
+    def __eq__(self, o) -> bool:
+        return self is o or (isinstance(o, _Value) and self._h == o._h and self._v == o._v)
+
+
 class Bond:
-    """A leg: type (ket -1 / bra +1 / regular 0), qnums [nq][nsym], degeneracies, symmetries."""
+    """A leg: type (ket -1 / bra +1 / regular 0), qnums [nq][nsym], degeneracies, symmetries.
+    A bond never changes once made (its tables are read-only), so copies share them."""
 
     def __init__(self, *args, **kw):
         # Bond(dim) | Bond(dim, type) | Bond(type, qnums, degs, syms=None)
@@ -145,15 +165,16 @@ class Bond:
             self._qnums = np.zeros((0, 0), dtype=np.int64)
             self._degs = np.zeros(0, dtype=np.int64)
             self._syms: List[Symmetry] = []
+            self._seal()
             return
         btype, qnums, degs = args[0], args[1], args[2]
         syms = args[3] if len(args) > 3 else kw.get("syms", None)
         self._type = int(btype)
-        q = np.asarray(qnums, dtype=np.int64)
+        q = np.array(qnums, dtype=np.int64)
         if q.ndim == 1:
             q = q.reshape(-1, 1)
         self._qnums = q
-        self._degs = np.asarray(degs, dtype=np.int64)
+        self._degs = np.array(degs, dtype=np.int64)
         if len(self._degs) != len(self._qnums):
             raise CytnxError("[Bond] qnums and degs must have the same length")
         if syms is None:
@@ -163,6 +184,12 @@ class Bond:
             if s.stype == 0 and ((col < 0) | (col >= s.n)).any():
                 raise CytnxError(f"[Bond] qnum out of range for {s.stype_str()}")
         self._dim = int(self._degs.sum())
+        self._seal()
+
+    def _seal(self) -> None:
+        self._qnums.setflags(write=False)
+        self._degs.setflags(write=False)
+        self._idc = self._secc = None
 
     # accessors (include/Bond.hpp)
     def dim(self) -> int:
@@ -189,12 +216,14 @@ class Bond:
     def redirect(self) -> "Bond":
         b = self.clone()
         b._type = -self._type
+        b._idc = None
         return b
 
     def clone(self) -> "Bond":
         b = Bond.__new__(Bond)
         b._dim, b._type = self._dim, self._type
-        b._qnums, b._degs, b._syms = self._qnums.copy(), self._degs.copy(), list(self._syms)
+        b._qnums, b._degs, b._syms = self._qnums, self._degs, self._syms
+        b._idc, b._secc = self._idc, self._secc
         return b
 
     def __eq__(self, o) -> bool:
@@ -208,9 +237,18 @@ class Bond:
             return f"Bond(dim={self._dim}, {t})"
         return f"Bond({t}, qnums={self.qnums()}, degs={self.getDegeneracies()})"
 
-    def _sig(self):
-        return (self._type, self._dim, self._qnums.tobytes(), self._degs.tobytes(),
-                tuple((s.stype, s.n) for s in self._syms))
+    def _id(self) -> _Value:
+        """The bond's value as a key."""
+        if self._idc is None:
+            self._idc = _Value((self._type, self._dim, self._qnums.tobytes(), self._degs.tobytes(),
+                                tuple((s.stype, s.n) for s in self._syms)))
+        return self._idc
+
+    def _sectors(self) -> _Value:
+        """Its charges and degeneracies as a key."""
+        if self._secc is None:
+            self._secc = _Value((self._qnums.shape, self._qnums.tobytes(), self._degs.tobytes()))
+        return self._secc
 
 
 def enumerate_blocks(bonds: Sequence[Bond]) -> np.ndarray:
@@ -236,23 +274,26 @@ def enumerate_blocks(bonds: Sequence[Bond]) -> np.ndarray:
 
 
 # ---------------------------------------------------------------- Tensor
-def _u64(a):
-    return np.ascontiguousarray(np.asarray(a, dtype=np.uint64))
-
-
 def device_permute(src: torch.Tensor, old_shape: Sequence[int], mapper: Sequence[int]) -> torch.Tensor:
     """out = src (row-major, old_shape) permuted by mapper, on the device (ctn_permute)."""
     require_cuda(src, "permute")
-    n = int(np.prod(old_shape)) if len(old_shape) else 1
+    n = math.prod(old_shape)
     out = torch.empty(n, dtype=src.dtype, device=src.device)
     if n == 0:
         return out
-    dt = Type.from_torch(src.dtype)
-    shp, mp = _u64(old_shape), _u64(mapper)
-    _lib.check(_lib.lib().ctn_permute(src.data_ptr(), out.data_ptr(), dt, len(old_shape),
-                                      shp.ctypes.data_as(_lib.P_u64), mp.ctypes.data_as(_lib.P_u64),
-                                      _lib.stream_ptr()), "Tensor::contiguous")
+    _lib.check(_lib.lib().ctn_permute(src.data_ptr(), out.data_ptr(),
+                                      *_permute_args(src.dtype, tuple(old_shape), tuple(mapper)), _lib.stream_ptr()),
+               "Tensor::contiguous")
     return out
+
+
+@functools.lru_cache(maxsize=1024)
+def _permute_args(dtype: torch.dtype, old_shape: tuple, mapper: tuple) -> tuple:
+    """dtype id, rank, shape and mapper as ctn_permute takes them (building them costs more than
+    the call)."""
+    r = len(old_shape)
+    return (Type.from_torch(dtype), r, (ctypes.c_uint64 * max(r, 1))(*old_shape),
+            (ctypes.c_uint64 * max(r, 1))(*mapper))
 
 
 class Tensor:
@@ -278,6 +319,17 @@ class Tensor:
         out._shape = list(t.shape)
         out._mapper = list(range(t.dim()))
         out._invmapper = list(range(t.dim()))
+        out._contiguous = True
+        return out
+
+    @staticmethod
+    def _wrap(flat: torch.Tensor, shape: Sequence[int]) -> "Tensor":
+        """A contiguous tensor of `shape` over the 1-D storage `flat`."""
+        out = Tensor.__new__(Tensor)
+        out._storage = flat
+        out._shape = list(shape)
+        out._mapper = list(range(len(out._shape)))
+        out._invmapper = list(out._mapper)
         out._contiguous = True
         return out
 
@@ -354,7 +406,7 @@ class Tensor:
         """Tensor_impl::contiguous (include/backend/Tensor_impl.hpp:222-254)."""
         if self._contiguous:
             return self
-        old_shape = [self._shape[self._invmapper[i]] for i in range(len(self._shape))]
+        old_shape = [self._shape[i] for i in self._invmapper]
         out = Tensor.__new__(Tensor)
         out._storage = device_permute(self._storage, old_shape, self._mapper)
         out._shape = list(self._shape)

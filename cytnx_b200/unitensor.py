@@ -16,6 +16,7 @@ one grouped-GEMM launch per call (cytnx_b200/csrc/blocks.cpp, gemm_f64.cu).
 from __future__ import annotations
 
 import ctypes
+import math
 from typing import Dict, List, Optional, Sequence, Tuple, Union
 
 import numpy as np
@@ -64,7 +65,7 @@ _LAYOUTS: Dict[tuple, BlockLayout] = {}
 
 
 def layout_for(bonds: Sequence[Bond]) -> BlockLayout:
-    key = tuple(b._sig() for b in bonds)
+    key = tuple([b._id() for b in bonds])
     lay = _LAYOUTS.get(key)
     if lay is None:
         lay = BlockLayout(bonds)
@@ -172,7 +173,6 @@ class UniTensor:
             r = len(self._bonds)
             self._labels = [str(l) for l in labels] if labels else [str(i) for i in range(r)]
             self._rowrank = (1 if self._is_diag else (r // 2 if r else 0)) if rowrank < 0 else int(rowrank)
-            self._is_braket = False
             return
         bonds = list(args[0]) if args else []
         if len(args) > 1:
@@ -204,7 +204,6 @@ class UniTensor:
             self._layout = layout_for(self._bonds)
             self._mapper = list(range(r))
             self._data = torch.zeros(self._layout.nelem, dtype=Type.to_torch(dtype), device=Device.torch_device(dev))
-            self._is_braket = self._update_braket()
         else:
             if any(b.has_symmetry() for b in bonds):
                 raise CytnxError("[ERROR] cannot mix symmetric and regular bonds")
@@ -212,7 +211,6 @@ class UniTensor:
             shape = [b.dim() for b in bonds] if not self._is_diag else [bonds[0].dim()]
             self._block = Tensor(shape, dtype, dev)
             self._rowrank = (1 if self._is_diag else r // 2) if rowrank < 0 else int(rowrank)
-            self._is_braket = False
 
     # -------------------------------------------------------------- internal constructors
     @classmethod
@@ -227,7 +225,6 @@ class UniTensor:
         u._layout = layout
         u._mapper = list(mapper)
         u._data = data
-        u._is_braket = u._update_braket()
         return u
 
     @classmethod
@@ -240,10 +237,9 @@ class UniTensor:
         u._bonds = list(bonds)
         u._labels = list(labels)
         u._rowrank = int(rowrank)
-        u._is_braket = False
         return u
 
-    def _update_braket(self) -> bool:
+    def is_braket_form(self) -> bool:
         if self._kind != UTenType.Block:
             return False
         return all(b.type() == BD_KET for b in self._bonds[: self._rowrank]) and \
@@ -294,12 +290,9 @@ class UniTensor:
     def is_diag(self) -> bool:
         return self._is_diag
 
-    def is_braket_form(self) -> bool:
-        return self._is_braket
-
     def is_contiguous(self) -> bool:
         if self._kind == UTenType.Block:
-            return all(m == i for i, m in enumerate(self._mapper))
+            return self._mapper == list(range(len(self._mapper)))
         return self._block.is_contiguous()
 
     def syms(self) -> List[Symmetry]:
@@ -324,7 +317,6 @@ class UniTensor:
         if not (0 <= rowrank <= self.rank()):
             raise CytnxError("[ERROR] rowrank out of range")
         self._rowrank = int(rowrank)
-        self._is_braket = self._update_braket()
         return self
 
     def set_rowrank(self, rowrank: int) -> "UniTensor":
@@ -709,7 +701,7 @@ class UniTensor:
         u = self.contiguous()
         bonds = [{"type": b.type(), "nsym": b.Nsym(), "qnums": b._qnums, "degs": b._degs, "dim": b.dim(),
                   "syms": [{"stype": s.stype, "n": s.n} for s in b.syms()]} for b in u._bonds]
-        d = {"uten_type": u._kind, "is_braket_form": u._is_braket, "is_tag": u._kind == UTenType.Block,
+        d = {"uten_type": u._kind, "is_braket_form": u.is_braket_form(), "is_tag": u._kind == UTenType.Block,
              "is_diag": u._is_diag, "rowrank": u._rowrank, "name": u._name, "labels": u._labels,
              "bonds": bonds}
         if u._kind == UTenType.Block:
@@ -784,12 +776,12 @@ def Contract(A: UniTensor, B: UniTensor, cacheL: bool = False, cacheR: bool = Fa
     n1 = [i for i in range(A.rank()) if i not in c1]
     n2 = [i for i in range(B.rank()) if i not in c2]
     if A._kind == UTenType.Block:
-        if A.syms() != B.syms():
+        if (A._bonds[0]._syms if A._bonds else []) != (B._bonds[0]._syms if B._bonds else []):
             raise CytnxError("[ERROR][BlockUniTensor][contract] Two UniTensor have different symmetry types, cannot contract.")
         for l, i, j in zip(comm, c1, c2):
-            if A._bonds[i].type() + B._bonds[j].type() != 0:
+            if A._bonds[i]._type + B._bonds[j]._type != 0:
                 raise CytnxError(f"[ERROR][BlockUniTensor][contract] A bond with type BRA can only be contracted with type KET. Invalid contraction for label '{l}'.")
-            if not (np.array_equal(A._bonds[i]._qnums, B._bonds[j]._qnums) and np.array_equal(A._bonds[i]._degs, B._bonds[j]._degs)):
+            if A._bonds[i]._sectors() != B._bonds[j]._sectors():
                 raise CytnxError(f"[ERROR][BlockUniTensor][contract] Contracted bond with label '{l}' has a qnum/degeneracy mismatch.")
     else:
         for l, i, j in zip(comm, c1, c2):
@@ -799,7 +791,7 @@ def Contract(A: UniTensor, B: UniTensor, cacheL: bool = False, cacheR: bool = Fa
         return _outer(A, B)
     if not n1 and not n2:
         return _full_contract(A, B, c1, c2)
-    out_bonds = [A._bonds[i].clone() for i in n1] + [B._bonds[i].clone() for i in n2]
+    out_bonds = [A._bonds[i] for i in n1] + [B._bonds[i] for i in n2]
     out_labels = [A._labels[i] for i in n1] + [B._labels[i] for i in n2]
     out_rowrank = A._rowrank + B._rowrank - sum(1 for i in c1 if i < A._rowrank) - sum(1 for i in c2 if i < B._rowrank)
     dtA, dtB = A._storage_tensor().dtype, B._storage_tensor().dtype
@@ -837,10 +829,9 @@ def Contract(A: UniTensor, B: UniTensor, cacheL: bool = False, cacheR: bool = Fa
         dO = BlockDesc(len(out_shape), 1, it.ctypes.data, sh.ctypes.data, of.ctypes.data, None)
         plan = _make_plan(dA, dB, c1, c2, dO, keep)
         _PLANS[key] = plan
-    out = torch.empty(int(np.prod(out_shape)), dtype=torch.float64, device=A._block._storage.device)
+    out = torch.empty(math.prod(out_shape), dtype=torch.float64, device=A._block._storage.device)
     _run_plan(plan, A._block._storage, B._block._storage, out)
-    blk = Tensor.from_torch(out.view(*out_shape))
-    return UniTensor._new_dense(blk, out_bonds, out_labels, out_rowrank)
+    return UniTensor._new_dense(Tensor._wrap(out, out_shape), out_bonds, out_labels, out_rowrank)
 
 
 def _make_plan(dA, dB, c1, c2, dO, keep) -> _ContractPlan:
@@ -854,9 +845,11 @@ def _make_plan(dA, dB, c1, c2, dO, keep) -> _ContractPlan:
 
 
 def _run_plan(plan: _ContractPlan, a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> None:
-    scratch = torch.empty(max(plan.scratch, 16), dtype=torch.uint8, device=a.device)
+    # 256 bytes: no operand is staged, and the scratch is not touched
+    scratch = torch.empty(plan.scratch, dtype=torch.uint8, device=a.device) if plan.scratch > 256 else None
     _lib.check(_lib.lib().ctn_contract_execute(plan.h, 3, a.data_ptr(), b.data_ptr(), out.data_ptr(),
-                                               scratch.data_ptr(), _lib.stream_ptr()), "contract")
+                                               None if scratch is None else scratch.data_ptr(), _lib.stream_ptr()),
+               "contract")
 
 
 def contract_plan_flops(A: UniTensor, B: UniTensor) -> float:
@@ -888,7 +881,6 @@ def structure_only(bonds: Sequence[Bond], labels: Sequence[str], rowrank: int = 
     u._layout = layout_for(u._bonds)
     u._mapper = list(range(len(bonds)))
     u._data = torch.empty(0, dtype=torch.float64)
-    u._is_braket = u._update_braket()
     return u
 
 
