@@ -40,38 +40,65 @@ struct VecHash {
 };
 using Key = std::vector<int64_t>;
 
-constexpr int MPO_CHUNK = 2048;
+// X3 block = sum of its X1 blocks times their coefficients, in chunks of MPO_CHUNK elements, one CTA
+// each.  Bound by HBM at D=4096 (X1 read and X3 written once: 201 MB) and by latency below: a chunk
+// carries its offsets and first two terms (all that most blocks have), so the X1 loads wait on one
+// descriptor, and a thread's loads of both terms are in flight together.  X1 and X3 blocks start
+// on 16-byte boundaries when the workspace does (VEC).  One chunk per CTA behind its block's own
+// descriptor, 8-byte loads, before: D=4096 59 -> 41 us, D=1024 10.7 -> 8.4 us.
+constexpr int MPO_CHUNK = 1024, MPO_THREADS = 256;
 
-__global__ void __launch_bounds__(256) k_mpo_apply(const double *__restrict__ X1, double *__restrict__ X3,
-                                                   const MpoTask *__restrict__ tasks,
-                                                   const MpoTerm *__restrict__ terms,
-                                                   const MpoChunk *__restrict__ chunks, int64_t nchunks) {
-  // each thread owns MPO_CHUNK / 256 elements of the chunk, 256 apart; the terms run outside
-  // so a term's loads for all of them are in flight together (per element the sum order over
-  // the terms is unchanged)
-  constexpr int PER = MPO_CHUNK / 256;
-  for (int64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-    const MpoChunk ch = chunks[c];
-    const MpoTask tk = tasks[ch.task];
-    const int64_t end = tk.size < ch.start + MPO_CHUNK ? tk.size : ch.start + MPO_CHUNK;
-    const int64_t e0 = ch.start + threadIdx.x;
-    double s[PER];
+template <bool VEC>
+__global__ void __launch_bounds__(MPO_THREADS) k_mpo_apply(const double *__restrict__ X1, double *__restrict__ X3,
+                                                           const MpoTerm *__restrict__ terms,
+                                                           const MpoChunk *__restrict__ chunks) {
+  constexpr int W = VEC ? 2 : 1;                      // elements per access
+  constexpr int PER = MPO_CHUNK / MPO_THREADS / W;    // accesses per thread
+  const MpoChunk ch = chunks[blockIdx.x];
+  double s[PER][W];
 #pragma unroll
-    for (int j = 0; j < PER; ++j) s[j] = 0.0;
-    for (int t = 0; t < tk.term_count; ++t) {
-      const MpoTerm tm = terms[tk.term_begin + t];
-      const double *src = X1 + tm.x1_off;
+  for (int j = 0; j < PER; ++j)
 #pragma unroll
-      for (int j = 0; j < PER; ++j) {
-        const int64_t e = e0 + (int64_t)j * 256;
-        if (e < end) s[j] = fma(tm.coef, __ldg(src + e), s[j]);
-      }
-    }
+    for (int k = 0; k < W; ++k) s[j][k] = 0.0;
+  auto load = [&](const double *src, double (&v)[PER][W]) {
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
-      const int64_t e = e0 + (int64_t)j * 256;
-      if (e < end) X3[tk.x3_off + e] = s[j];
+      const int e = (threadIdx.x + j * MPO_THREADS) * W;
+      if (W == 2 && e + 1 < ch.len) {
+        const double2 x = __ldg(reinterpret_cast<const double2 *>(src + e));
+        v[j][0] = x.x;
+        v[j][W - 1] = x.y;
+      } else if (e < ch.len) {
+        v[j][0] = __ldg(src + e);
+        if (W == 2) v[j][W - 1] = 0.0;
+      } else {
+#pragma unroll
+        for (int k = 0; k < W; ++k) v[j][k] = 0.0;
+      }
     }
+  };
+  auto add = [&](double c, const double (&v)[PER][W]) {
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+#pragma unroll
+      for (int k = 0; k < W; ++k) s[j][k] = fma(c, v[j][k], s[j][k]);
+  };
+  double v0[PER][W], v1[PER][W];
+  load(X1 + ch.x1_off[0], v0);
+  if (ch.term_count > 1) load(X1 + ch.x1_off[1], v1);
+  add(ch.coef[0], v0);
+  if (ch.term_count > 1) add(ch.coef[1], v1);
+  for (int t = 2; t < ch.term_count; ++t) {
+    const MpoTerm tm = terms[ch.term_begin + t];
+    load(X1 + tm.x1_off + ch.start, v0);
+    add(tm.coef, v0);
+  }
+  double *o = X3 + ch.x3_off;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int e = (threadIdx.x + j * MPO_THREADS) * W;
+    if (W == 2 && e + 1 < ch.len) *reinterpret_cast<double2 *>(o + e) = make_double2(s[j][0], s[j][W - 1]);
+    else if (e < ch.len) o[e] = s[j][0];
   }
 }
 }  // namespace
@@ -82,16 +109,13 @@ ctn_status MpoApply::upload(cudaStream_t st) {
   if (d_mem && d_dev == dev) return CTN_OK;
   if (d_mem) cudaFree(d_mem);
   d_mem = nullptr;
-  const size_t bytes = tasks.size() * sizeof(MpoTask) + terms.size() * sizeof(MpoTerm) +
-                       chunks.size() * sizeof(MpoChunk) + 64;
+  const size_t bytes = chunks.size() * sizeof(MpoChunk) + terms.size() * sizeof(MpoTerm) + 64;
   CTN_CUDA(cudaMalloc(&d_mem, bytes));
   d_dev = dev;
   char *p = (char *)d_mem;
-  if (!tasks.empty()) CTN_CUDA(cudaMemcpyAsync(p, tasks.data(), tasks.size() * sizeof(MpoTask), cudaMemcpyHostToDevice, st));
-  p += tasks.size() * sizeof(MpoTask);
-  if (!terms.empty()) CTN_CUDA(cudaMemcpyAsync(p, terms.data(), terms.size() * sizeof(MpoTerm), cudaMemcpyHostToDevice, st));
-  p += terms.size() * sizeof(MpoTerm);
   if (!chunks.empty()) CTN_CUDA(cudaMemcpyAsync(p, chunks.data(), chunks.size() * sizeof(MpoChunk), cudaMemcpyHostToDevice, st));
+  p += chunks.size() * sizeof(MpoChunk);
+  if (!terms.empty()) CTN_CUDA(cudaMemcpyAsync(p, terms.data(), terms.size() * sizeof(MpoTerm), cudaMemcpyHostToDevice, st));
   CTN_CUDA(cudaStreamSynchronize(st));
   return CTN_OK;
 }
@@ -99,15 +123,13 @@ ctn_status MpoApply::upload(cudaStream_t st) {
 ctn_status MpoApply::run(const double *X1, double *X3, cudaStream_t st) {
   CTN_TRY(upload(st));
   if (chunks.empty()) return CTN_OK;
-  const char *p = (const char *)d_mem;
-  const MpoTask *dt = (const MpoTask *)p;
-  const MpoTerm *dm = (const MpoTerm *)(p + tasks.size() * sizeof(MpoTask));
-  const MpoChunk *dc = (const MpoChunk *)(p + tasks.size() * sizeof(MpoTask) + terms.size() * sizeof(MpoTerm));
-  int dev = 0, nsm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t grid = std::min<int64_t>((int64_t)chunks.size(), (int64_t)nsm * 8);
-  k_mpo_apply<<<(unsigned)grid, 256, 0, st>>>(X1, X3, dt, dm, dc, (int64_t)chunks.size());
+  const MpoChunk *dc = (const MpoChunk *)d_mem;
+  const MpoTerm *dm = (const MpoTerm *)(dc + chunks.size());
+  const unsigned grid = (unsigned)chunks.size();
+  if (((reinterpret_cast<uintptr_t>(X1) | reinterpret_cast<uintptr_t>(X3)) & 15) == 0)
+    k_mpo_apply<true><<<grid, MPO_THREADS, 0, st>>>(X1, X3, dm, dc);
+  else
+    k_mpo_apply<false><<<grid, MPO_THREADS, 0, st>>>(X1, X3, dm, dc);
   CTN_CHECK_LAUNCH();
   return CTN_OK;
 }
@@ -116,7 +138,20 @@ void MpoApply::finalize() {
   chunks.clear();
   bytes = 0.0;
   for (size_t t = 0; t < tasks.size(); ++t) {
-    for (int64_t s = 0; s < tasks[t].size; s += MPO_CHUNK) chunks.push_back({(int32_t)t, 0, s});
+    const MpoTask &tk = tasks[t];
+    for (int64_t s = 0; s < tk.size; s += MPO_CHUNK) {
+      MpoChunk c{};
+      c.x3_off = tk.x3_off + s;
+      c.start = s;
+      c.len = (int32_t)std::min<int64_t>(MPO_CHUNK, tk.size - s);
+      c.term_begin = tk.term_begin;
+      c.term_count = tk.term_count;
+      for (int k = 0; k < 2 && k < tk.term_count; ++k) {
+        c.x1_off[k] = terms[tk.term_begin + k].x1_off + s;
+        c.coef[k] = terms[tk.term_begin + k].coef;
+      }
+      chunks.push_back(c);
+    }
     bytes += 8.0 * tasks[t].size * (1 + tasks[t].term_count);
   }
 }
@@ -270,7 +305,7 @@ extern "C" ctn_status ctn_heff2_plan_create(const ctn_heff2_desc *d, ctn_heff2_p
         x3_terms.push_back(terms);
         x3_or.push_back({o, r});
         mtasks.push_back(mt);
-        p->x3_elems += rows * cols;
+        p->x3_elems += (rows * cols + 1) / 2 * 2;  // blocks start on 16-byte boundaries
       }
       GemmPairD pr;
       pr.a_off = xt->second;
@@ -317,7 +352,7 @@ extern "C" ctn_status ctn_heff2_plan_create(const ctn_heff2_desc *d, ctn_heff2_p
     pr.flags = 1;
     p->g1.pairs.push_back(pr);
     p->g1.tasks.push_back(tk);
-    p->x1_elems += M * N;
+    p->x1_elems += (M * N + 1) / 2 * 2;
   }
   // resolve term offsets
   {
@@ -379,7 +414,7 @@ extern "C" size_t ctn_heff2_psi_elems(const ctn_heff2_plan *p) { return (size_t)
 static int split_kind(int precision) { return precision == CTN_PREC_BF16X3 ? ctn::TC_BF16 : ctn::TC_TF32; }
 
 extern "C" size_t ctn_heff2_workspace_bytes(const ctn_heff2_plan *p, int precision) {
-  if (precision == CTN_PREC_F64) return (size_t)(p->L_elems + p->x1_elems + p->x3_elems) * sizeof(double) + 256;
+  if (precision == CTN_PREC_F64) return (size_t)(p->L_elems + 1 + p->x1_elems + p->x3_elems) * sizeof(double) + 256;
   if (precision != CTN_PREC_3XTF32 && precision != CTN_PREC_BF16X3) return 0;
   auto *pp = const_cast<ctn_heff2_plan *>(p);
   if (ctn::heff_split_prepare(pp, split_kind(precision)) != CTN_OK) return 0;
@@ -418,7 +453,7 @@ extern "C" ctn_status ctn_heff2_matvec(ctn_heff2_plan *p, const double *psi, dou
   CTN_REQUIRE(precision == CTN_PREC_F64, "ctn_heff2_matvec: unknown precision %d", precision);
   CTN_REQUIRE(p->bound, "ctn_heff2_matvec: environments not bound (call ctn_heff2_set_env)");
   double *Lt = p->ws;
-  double *X1 = Lt + p->L_elems;
+  double *X1 = Lt + (p->L_elems + 1) / 2 * 2;
   double *X3 = X1 + p->x1_elems;
   CTN_TRY(p->g1.run(Lt, psi, X1, st));
   CTN_TRY(p->mpo.run(X1, X3, st));
@@ -538,7 +573,7 @@ extern "C" ctn_status ctn_heff2_profile(ctn_heff2_plan *p, const double *psi, do
   }
   CTN_REQUIRE(p->bound, "ctn_heff2_profile: environments not bound");
   double *Lt = p->ws;
-  double *X1 = Lt + p->L_elems;
+  double *X1 = Lt + (p->L_elems + 1) / 2 * 2;
   double *X3 = X1 + p->x1_elems;
   // warm the table uploads outside the timed region
   CTN_TRY(p->g1.upload(st));

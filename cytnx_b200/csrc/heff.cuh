@@ -14,10 +14,12 @@ struct MpoTerm {
   int64_t x1_off;
   double coef;
 };
-struct MpoChunk {
-  int32_t task;
-  int32_t pad_;
-  int64_t start;
+// a run of at most 1024 elements of an X3 block with its first two terms
+struct alignas(16) MpoChunk {
+  int64_t x3_off, start;   // first element in X3 and inside the block
+  int64_t x1_off[2];       // of the first two terms, at that element
+  double coef[2];
+  int32_t len, term_begin, term_count, pad_;
 };
 struct MpoApply {
   std::vector<MpoTask> tasks;
