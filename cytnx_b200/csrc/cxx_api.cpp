@@ -1222,6 +1222,11 @@ int matvec_cb(void *user, const double *x, double *y, void *stream) {
     return 1;
   }
 }
+
+// bytes of ctn_lanczos_gnd's work buffer
+size_t gnd_work_bytes(int64_t n, unsigned int maxiter) {
+  return (size_t)std::max<int64_t>(4 * n + 64, n + 1104 + (int64_t)maxiter) * 8;
+}
 }  // namespace
 
 std::vector<UniTensor> Lanczos(LinOp *Hop, const UniTensor &Tin, const std::string method, const double &CvgCrit,
@@ -1237,7 +1242,7 @@ std::vector<UniTensor> Lanczos(LinOp *Hop, const UniTensor &Tin, const std::stri
     throw error("[ERROR][Lanczos] the LinOp's nx does not match the initial vector.");
   const int dev = tmpl.device();
   const unsigned int maxiter = std::max(1u, Maxiter);
-  detail::DevBuf kry((size_t)(maxiter + 1) * n * 8, dev, false), work((size_t)(4 * n + 64) * 8, dev, false);
+  detail::DevBuf kry((size_t)(maxiter + 1) * n * 8, dev, false), work(gnd_work_bytes(n, maxiter), dev, false);
   UniTensor vec = tmpl.clone();
   CbCtx ctx;
   ctx.op = Hop;
@@ -1267,7 +1272,7 @@ std::vector<Tensor> Lanczos(LinOp *Hop, const Tensor &Tin, const std::string met
   if (Hop->nx() && (int64_t)Hop->nx() != n) throw error("[ERROR][Lanczos] the LinOp's nx does not match Tin.");
   const int dev = tmpl.device();
   const unsigned int maxiter = std::max(1u, Maxiter);
-  detail::DevBuf kry((size_t)(maxiter + 1) * n * 8, dev, false), work((size_t)(4 * n + 64) * 8, dev, false);
+  detail::DevBuf kry((size_t)(maxiter + 1) * n * 8, dev, false), work(gnd_work_bytes(n, maxiter), dev, false);
   Tensor vec(tmpl.shape(), Type.Double, dev, false);
   CbCtx ctx;
   ctx.op = Hop;

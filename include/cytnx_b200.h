@@ -326,7 +326,8 @@ void ctn_heff2_batch_destroy(ctn_heff2_batch *batch);
 /* ---------------------------------------------------------------- Lanczos
  * Ground state by the Lanczos_Gnd_Ut recurrence on flat FP64 device vectors.
  * matvec(user, x, y, stream) must write y = H x on `stream`.  krylov must hold
- * (maxiter + 1) * n doubles (device); work >= 4 * n + 64 doubles (device).
+ * (maxiter + 1) * n doubles (device); work >= max(4 * n + 64, n + 1104 + maxiter) doubles
+ * (device): the vector, 8 scalars, the reductions' 1032 and the Ritz coefficients.
  * On return *energy holds the lowest Ritz value, eigvec (device, n) the Ritz
  * vector, *iters the iterations done.  Semantics follow the reference: stop
  * when |E_i - E_{i-1}| < cvgcrit or beta == 0 or maxiter reached; matvec is called exactly
