@@ -191,6 +191,14 @@ class Bond:
         self._degs.setflags(write=False)
         self._idc = self._secc = None
 
+    # the keys stay behind: they hold hashes of bytes, which differ from process to process
+    def __getstate__(self) -> dict:
+        return {k: v for k, v in self.__dict__.items() if k not in ("_idc", "_secc")}
+
+    def __setstate__(self, state: dict) -> None:
+        self.__dict__.update(state)
+        self._seal()
+
     # accessors (include/Bond.hpp)
     def dim(self) -> int:
         return self._dim
