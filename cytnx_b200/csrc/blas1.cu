@@ -504,7 +504,8 @@ template <bool VEC, typename WT>
 __global__ void __launch_bounds__(RT, 4) k_lanczos_gnd_step(const WT *__restrict__ w, const double *__restrict__ p1,
                                                             const double *__restrict__ p0, double *dst, int64_t n,
                                                             const double *beta, double *out_alpha, double *out_beta,
-                                                            double *ws, unsigned *err, long long spins) {
+                                                            double *ws, unsigned *err, unsigned extra,
+                                                            long long spins) {
   __shared__ double coef;
   const int64_t tid = (int64_t)blockIdx.x * RT + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * RT;
@@ -546,7 +547,7 @@ __global__ void __launch_bounds__(RT, 4) k_lanczos_gnd_step(const WT *__restrict
   for (int64_t i = 2 * n2 + tid; i < n; i += step) s = fma((double)w[i], p1[i], s);
   s = block_sum(s);
   if (threadIdx.x == 0) ws[blockIdx.x] = s;
-  if (!grid_barrier(bar, bar + 1, 0u, spins)) return gave_up();
+  if (!grid_barrier(bar, bar + 1, extra, spins)) return gave_up();
   const double a = total(ws);
   // ---- v and its norm
   const double b = p0 ? *beta : 0.0;
@@ -573,7 +574,7 @@ __global__ void __launch_bounds__(RT, 4) k_lanczos_gnd_step(const WT *__restrict
   for (int64_t i = 2 * n2 + tid; i < n; i += step) dst[i] = one((double)w[i], p1[i], p0 ? p0[i] : 0.0);
   s = block_sum(s);
   if (threadIdx.x == 0) ws[GND_CTAS + blockIdx.x] = s;
-  if (!grid_barrier(bar, bar + 1, 0u, spins)) return gave_up();
+  if (!grid_barrier(bar, bar + 1, extra, spins)) return gave_up();
   const double nrm = sqrt(total(ws + GND_CTAS));
   if (tid == 0) {
     *out_alpha = a;
@@ -858,10 +859,10 @@ ctn_status krylov_step_f64(const float *w, const double *u, const double *up, co
 template <typename WT>
 static ctn_status lanczos_gnd_step_any(const WT *w, const double *p1, const double *p0, double *dst, int64_t n,
                                        const double *beta, double *out_alpha, double *out_beta, double *ws,
-                                       unsigned *err, cudaStream_t st) {
+                                       unsigned *err, cudaStream_t st, unsigned extra, long long spins) {
   const bool vec = aligned16(w) && aligned16(p1) && aligned16(dst) && (!p0 || aligned16(p0));
   void (*kern)(const WT *, const double *, const double *, double *, int64_t, const double *, double *, double *,
-               double *, unsigned *, long long) = vec ? k_lanczos_gnd_step<true, WT> : k_lanczos_gnd_step<false, WT>;
+               double *, unsigned *, unsigned, long long) = vec ? k_lanczos_gnd_step<true, WT> : k_lanczos_gnd_step<false, WT>;
   // CTAs per SM that are resident together, queried once per device; 0 = no cooperative launch
   static int per_sm[64][2], sms[64];
   static bool known[64][2];
@@ -880,21 +881,21 @@ static ctn_status lanczos_gnd_step_any(const WT *w, const double *p1, const doub
   // at most three CTAs an SM: whole waves below GND_CTAS on 148 SMs
   const int most = std::min(GND_CTAS, sms[di] * std::min(3, per_sm[di][vec]));
   const int g = std::max(1, std::min(grid_stream(n), most));
-  long long spins = BARRIER_SPINS;
+  if (spins == 0) spins = BARRIER_SPINS;
   void *args[] = {(void *)&w,         (void *)&p1,       (void *)&p0, (void *)&dst, (void *)&n,    (void *)&beta,
-                  (void *)&out_alpha, (void *)&out_beta, (void *)&ws, (void *)&err, (void *)&spins};
+                  (void *)&out_alpha, (void *)&out_beta, (void *)&ws, (void *)&err, (void *)&extra, (void *)&spins};
   CTN_CUDA(cudaLaunchCooperativeKernel((const void *)kern, dim3(g), dim3(RT), args, 0, st));
   return CTN_OK;
 }
 ctn_status lanczos_gnd_step_f64(const double *w, const double *p1, const double *p0, double *dst, int64_t n,
                                 const double *beta, double *out_alpha, double *out_beta, double *ws, unsigned *err,
-                                cudaStream_t st) {
-  return lanczos_gnd_step_any(w, p1, p0, dst, n, beta, out_alpha, out_beta, ws, err, st);
+                                cudaStream_t st, unsigned extra, long long spins) {
+  return lanczos_gnd_step_any(w, p1, p0, dst, n, beta, out_alpha, out_beta, ws, err, st, extra, spins);
 }
 ctn_status lanczos_gnd_step_f64(const float *w, const double *p1, const double *p0, double *dst, int64_t n,
                                 const double *beta, double *out_alpha, double *out_beta, double *ws, unsigned *err,
-                                cudaStream_t st) {
-  return lanczos_gnd_step_any(w, p1, p0, dst, n, beta, out_alpha, out_beta, ws, err, st);
+                                cudaStream_t st, unsigned extra, long long spins) {
+  return lanczos_gnd_step_any(w, p1, p0, dst, n, beta, out_alpha, out_beta, ws, err, st, extra, spins);
 }
 
 ctn_status div_copy_f64(const double *x, double *y, int64_t n, const double *a, cudaStream_t st) {

@@ -45,14 +45,15 @@ ctn_status krylov_step_f64(const float *w, const double *u, const double *up, co
 // one step of the plain recurrence in one cooperative launch: *out_alpha = <w, p1>, v = w - alpha p1 -
 // *beta p0 (p0 may be null), *out_beta = |v|, dst = v / |v|; ws: the reduction workspace (zeroed
 // before its first use).  A barrier wait that runs out sets *err (device word, zeroed by the
-// caller) and alpha and beta to NaN.  CTN_ERR_UNSUPPORTED without launching when the device has
+// caller) and alpha and beta to NaN; extra: arrivals the barriers wait for beyond the grid's, spins: probes
+// of a wait, 0 for the usual limit (both for the self-test).  CTN_ERR_UNSUPPORTED without launching when the device has
 // no cooperative launch.
 ctn_status lanczos_gnd_step_f64(const double *w, const double *p1, const double *p0, double *dst, int64_t n,
                                 const double *beta, double *out_alpha, double *out_beta, double *ws, unsigned *err,
-                                cudaStream_t st);
+                                cudaStream_t st, unsigned extra = 0, long long spins = 0);
 ctn_status lanczos_gnd_step_f64(const float *w, const double *p1, const double *p0, double *dst, int64_t n,
                                 const double *beta, double *out_alpha, double *out_beta, double *ws, unsigned *err,
-                                cudaStream_t st);
+                                cudaStream_t st, unsigned extra = 0, long long spins = 0);
 ctn_status div_copy_f64(const double *x, double *y, int64_t n, const double *a, cudaStream_t st);
 ctn_status combine_f64(const double *K, int64_t n, int m, const double *c, double *out, cudaStream_t st);
 // block Krylov helpers (basis V: m vectors of n doubles back to back)

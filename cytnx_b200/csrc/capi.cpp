@@ -192,7 +192,8 @@ static ctn_status pinned_scalars(double **out) {
 // without side effects.
 ctn_status lanczos_gnd(int (*mv)(void *, const double *, double *, void *), void *user, const double *psi0,
                        int64_t n, int maxiter, double cvgcrit, double *krylov, double *work, double *eigvec,
-                       double *energy, int *iters, cudaStream_t st, bool speculate, bool w_f32) {
+                       double *energy, int *iters, cudaStream_t st, bool speculate, bool w_f32,
+                       unsigned barrier_extra, long long barrier_spins) {
   CTN_REQUIRE(maxiter >= 2, "[Lanczos] Maxiter must >1");
   CTN_REQUIRE(cvgcrit > 0, "[Lanczos] converge criteria must >0");
   CTN_REQUIRE(n > 0, "[Lanczos] empty vector");
@@ -239,8 +240,11 @@ ctn_status lanczos_gnd(int (*mv)(void *, const double *, double *, void *), void
     if (mv(user, pi, w, st) != 0) return CTN_ERR_CUDA;
     const float *wf = reinterpret_cast<const float *>(w);
     if (fused) {
-      const ctn_status r = w_f32 ? lanczos_gnd_step_f64(wf, pi, po, pi + n, n, b_old, scal + 1, b_new, ws, err, st)
-                                 : lanczos_gnd_step_f64(w, pi, po, pi + n, n, b_old, scal + 1, b_new, ws, err, st);
+      auto step = [&](const auto *wv) {
+        return lanczos_gnd_step_f64(wv, pi, po, pi + n, n, b_old, scal + 1, b_new, ws, err, st, barrier_extra,
+                                    barrier_spins);
+      };
+      const ctn_status r = w_f32 ? step(wf) : step(w);
       if (r == CTN_ERR_UNSUPPORTED) fused = false;  // found in iteration 0, nothing launched
       else CTN_TRY(r);
     }
@@ -258,6 +262,12 @@ ctn_status lanczos_gnd(int (*mv)(void *, const double *, double *, void *), void
   std::vector<double> As, Bs, evals, evecs;
   double E = 0.0;
   int it = 0;
+  // an error leaves the iteration that was queued ahead behind: it writes the caller's buffers and this
+  // thread's pinned slots, so nothing returns before the stream has run dry
+  struct Drain {
+    cudaStream_t st;
+    ~Drain() { cudaStreamSynchronize(st); }
+  } drain{st};
   CTN_TRY(queue(0));
   for (int i = 0; i < maxiter; ++i) {
     it = i + 1;
@@ -266,7 +276,9 @@ ctn_status lanczos_gnd(int (*mv)(void *, const double *, double *, void *), void
     if (speculate && i + 1 < maxiter) CTN_TRY(queue(i + 1));
     CTN_CUDA(cudaEventSynchronize(ev[i & 1]));
     const double alpha = pin[4 * (i & 1)], beta = pin[4 * (i & 1) + 1 + (i & 1)];
-    if (pin[4 * (i & 1) + 3] != 0.0) {
+    unsigned gave_up;  // the error word; as a double it would be a denormal, zero to a thread that flushes them
+    std::memcpy(&gave_up, pin + 4 * (i & 1) + 3, sizeof(gave_up));
+    if (gave_up) {
       set_error("[Lanczos] the grid barrier of a fused step gave up waiting");
       return CTN_ERR_TIMEOUT;
     }
@@ -448,6 +460,51 @@ extern "C" ctn_status ctn_lanczos_gnd(ctn_matvec_fn matvec, void *user, const do
                                       int *iters, void *stream) {
   return ctn::lanczos_gnd(matvec, user, psi0, n, maxiter, cvgcrit, krylov, work, eigvec, energy, iters,
                           ctn::as_stream(stream), /*speculate=*/false, /*w_f32=*/false);
+}
+
+// Self-test of the give-up path of lanczos_gnd: the identity as the operator, barriers that wait for one
+// arrival more than the grid has.
+namespace ctn {
+static int identity_mv(void *n, const double *x, double *y, void *stream) {
+  return cudaMemcpyAsync(y, x, *(const size_t *)n * sizeof(double), cudaMemcpyDeviceToDevice, as_stream(stream)) ==
+                 cudaSuccess
+             ? 0
+             : 1;
+}
+static ctn_status selftest_lanczos_timeout(long long spin_limit, cudaStream_t st) {
+  constexpr int maxiter = 4;
+  size_t n = 1 << 14;
+  const size_t work = n + 1104 + maxiter, all = n + (maxiter + 1) * n + work + n;
+  double *buf = nullptr;
+  CTN_CUDA(cudaMalloc(&buf, all * sizeof(double)));
+  double *psi = buf, *kry = psi + n, *wk = kry + (maxiter + 1) * n, *eig = wk + work;
+  const double one = 1.0;
+  double energy = 0.0;
+  int iters = 0;
+  ctn_status rc = cudaMemsetAsync(buf, 0, all * sizeof(double), st) == cudaSuccess &&
+                          cudaMemcpyAsync(psi, &one, sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess
+                      ? CTN_OK
+                      : CTN_ERR_CUDA;
+  if (rc == CTN_OK)
+    rc = lanczos_gnd(identity_mv, &n, psi, (int64_t)n, maxiter, 1e-300, kry, wk, eig, &energy, &iters, st,
+                     /*speculate=*/true, /*w_f32=*/false, 1u, spin_limit);
+  const bool idle = cudaStreamQuery(st) == cudaSuccess;
+  cudaFree(buf);
+  if (rc == CTN_ERR_TIMEOUT && !idle) {
+    set_error("ctn_selftest_lanczos_timeout: the driver returned with work in flight");
+    return CTN_ERR_INVALID;
+  }
+  if (rc == CTN_OK) {
+    set_error("ctn_selftest_lanczos_timeout: the driver saw no error");
+    return CTN_ERR_INVALID;
+  }
+  return rc;
+}
+}  // namespace ctn
+
+extern "C" ctn_status ctn_selftest_lanczos_timeout(long long spin_limit, void *stream) {
+  CTN_REQUIRE(spin_limit > 0, "ctn_selftest_lanczos_timeout: spin_limit must be positive");
+  return ctn::selftest_lanczos_timeout(spin_limit, ctn::as_stream(stream));
 }
 
 namespace ctn {

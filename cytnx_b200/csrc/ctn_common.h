@@ -22,10 +22,12 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 
 // ground-state Lanczos (capi.cpp); speculate queues each next iteration before the host
 // solve of the current one (matvecs without side effects only: one extra call at the end);
-// w_f32: mv writes its result as n floats
+// w_f32: mv writes its result as n floats; barrier_extra, barrier_spins: of the fused step's barriers
+// (lanczos_gnd_step_f64), for the self-test
 ctn_status lanczos_gnd(int (*mv)(void *, const double *, double *, void *), void *user, const double *psi0,
                        int64_t n, int maxiter, double cvgcrit, double *krylov, double *work, double *eigvec,
-                       double *energy, int *iters, cudaStream_t st, bool speculate, bool w_f32);
+                       double *energy, int *iters, cudaStream_t st, bool speculate, bool w_f32,
+                       unsigned barrier_extra = 0, long long barrier_spins = 0);
 // restarted split-precision ground state (capi.cpp); w_f32: mv_lo writes its result as n floats
 ctn_status lanczos_refined(int (*mv_lo)(void *, const double *, double *, void *), void *u_lo,
                            int (*mv_hi)(void *, const double *, double *, void *), void *u_hi, const double *psi0,

@@ -222,6 +222,9 @@ ctn_status ctn_selftest_wait_timeout(int precision, long long spin_limit, void *
  * without cooperative launch); the context stays usable.  Allocates a small device buffer and
  * synchronises the stream.  No counterpart in the reference. */
 ctn_status ctn_selftest_barrier_timeout(long long spin_limit, void *stream);
+/* The same for the step of ctn_lanczos_gnd, through its driver with the next iteration queued ahead: the
+ * driver sees the error word, waits for what it has queued and returns CTN_ERR_TIMEOUT. */
+ctn_status ctn_selftest_lanczos_timeout(long long spin_limit, void *stream);
 
 /* ---------------------------------------------------------------- BLAS-1 (FP64)
  * Results of reductions land in device memory (out points to device doubles). */
