@@ -18,7 +18,8 @@
 //    of the input's fastest axis) x 128 tiles into shared memory with cp.async.bulk.tensor
 //    (SWIZZLE_128B, so the column reads of the transpose spread over the banks) and
 //    writes 16-byte vectors along the output's fastest axis.  A short output axis (< 16)
-//    under a long input axis has a staged kernel of its own.
+//    under a long input axis has a staged kernel of its own, and tensors whose tiles would be
+//    mostly empty go in boxes over any axes (permute_packed.cu).
 // No per-call allocation or host<->device copy of stride vectors: the reduced
 // geometry travels as kernel parameters (the reference mallocs and copies two
 // stride arrays per call, cuMovemem_gpu.cu:139-152).
@@ -33,12 +34,6 @@
 #include "tmap.h"
 
 namespace ctn {
-
-constexpr int kMaxRank = 16;
-
-struct alignas(16) U128 {
-  uint64_t a, b;
-};
 
 template <int N>
 struct VecT;
@@ -173,7 +168,8 @@ struct TransGeom {
 // of TA x TB elements: it reads runs of TA along A, stages them in shared memory and writes
 // runs of TB along B.  Grouping axes keeps the runs long when the last axes are short (a site
 // tensor's physical legs, a 37-element leg), and the tile's shape (powers of two, TA * TB = CAP)
-// follows the groups' extents, so few lanes idle on them.
+// follows the groups' extents.  A group ends where the next axis belongs to the other one: two short innermost
+// axes that are each other's neighbours leave most of a tile empty, and permute_packed takes such tensors.
 // These kernels are bound by instruction issue before HBM (a 32-lane access moves 32 elements of
 // a narrow type only), so a tile's shape is a compile-time constant: a row costs one offset and
 // one 64-bit multiply-add, an element its load, its store and the shared-memory round trip.  All
@@ -189,11 +185,6 @@ constexpr int TILE_THREADS = 256;
 constexpr int TILE_SMALL = 1024;
 constexpr int tile_cap(int es) { return es == 1 ? 8192 : es <= 4 ? 4096 : es == 8 ? 2048 : 1024; }
 constexpr int TILE_TA_MIN = 2, TILE_TA_MAX = 1024;  // tile widths along A (TB = CAP / TA likewise >= 2)
-// staged row pitch in elements: an odd number of 32-bit words (wider types: odd), so that the
-// column reads of consecutive b fall on different banks
-constexpr int tile_pitch(int es, int ta) {
-  return es >= 4 ? (ta | 1) : es == 2 ? (ta % 4 == 0 ? ta + 2 : ta) : (ta % 8 == 0 ? ta + 4 : ta);
-}
 
 template <int R, typename IT>
 struct TilePerm {
@@ -1009,6 +1000,11 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
   int64_t out_stride_of_old[kMaxRank];
   for (int i = 0; i < r; ++i) out_stride_of_old[rmap[i]] = out_stride[i];
   constexpr int WANT = ES == 1 ? 128 : 64;
+  // tiles that are mostly empty (short axes that are each other's neighbours, which neither group can join)
+  // give way to boxes over any axes
+  auto packed = [&](int64_t ntiles, int cap) {
+    return permute_packed(ES, src, dst, r, rshape, rmap, in_stride, out_stride_of_old, n, ntiles * cap, nsm, st);
+  };
   // 32-bit index arithmetic (a division costs several times less) when every offset fits
   if (n < ((int64_t)1 << 31)) {
     TilePerm<kMaxRank, uint32_t> g;
@@ -1016,8 +1012,10 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
     int64_t ntiles = tile_geometry(ES, tile_cap(ES), WANT, r, rshape, rmap, in_stride, out_stride_of_old, g);
     // fewer than two tiles per SM: the latency of one tile is all there is, so smaller tiles, and
     // axes joined only where a group would be very short (a joined group needs an offset table)
-    if (ntiles < 2 * nsm) {
-      ntiles = tile_geometry(ES, TILE_SMALL, 16, r, rshape, rmap, in_stride, out_stride_of_old, g);
+    const bool small = ntiles < 2 * nsm;
+    if (small) ntiles = tile_geometry(ES, TILE_SMALL, 16, r, rshape, rmap, in_stride, out_stride_of_old, g);
+    if (packed(ntiles, small ? TILE_SMALL : tile_cap(ES))) {
+    } else if (small) {
       launch_tile<T, TILE_SMALL>(src, dst, g, ntiles, st);
     } else {
       launch_tile<T, tile_cap(ES)>(src, dst, g, ntiles, st);
@@ -1026,7 +1024,7 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
     TilePerm<kMaxRank, uint64_t> g;
     g.src = g.dst = 0;
     const int64_t ntiles = tile_geometry(ES, tile_cap(ES), WANT, r, rshape, rmap, in_stride, out_stride_of_old, g);
-    launch_tile<T, tile_cap(ES)>(src, dst, g, ntiles, st);
+    if (!packed(ntiles, tile_cap(ES))) launch_tile<T, tile_cap(ES)>(src, dst, g, ntiles, st);
   }
   CTN_CHECK_LAUNCH();
   return CTN_OK;

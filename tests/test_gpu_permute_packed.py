@@ -1,0 +1,57 @@
+"""Permutes whose two innermost axes are short neighbours (boxes over any axes): exact against torch's own permute."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DTYPES = [torch.bool, torch.int16, torch.float32, torch.float64, torch.complex128]
+# neighbours on both sides with the same axis behind them, on both sides with different ones, on one side only;
+# axes cut into equal and unequal chunks on either side and on both; one box; boxes of several axes; planes wider
+# than half a tile's side; few elements (512 a box) and many
+CASES = [((9, 2, 2), (0, 2, 1)), ((5000, 2, 2), (0, 2, 1)), ((5001, 3, 5), (0, 2, 1)), ((70001, 2, 3), (0, 2, 1)),
+         ((300007, 2, 2), (0, 2, 1)), ((1201, 24, 24), (0, 2, 1)), ((7001, 10, 11), (0, 2, 1)),
+         ((257, 131, 2, 3), (1, 0, 3, 2)), ((1009, 613, 2, 3), (1, 0, 3, 2)), ((300, 301, 4, 8), (1, 0, 3, 2)),
+         ((601, 97, 4, 3), (3, 0, 2, 1)), ((601, 97, 4, 4, 3), (3, 1, 0, 4, 2)), ((1487, 4, 7, 16, 2), (0, 3, 1, 4, 2)),
+         ((59, 16, 5, 16, 12, 8), (1, 2, 3, 0, 5, 4)), ((155, 155, 4, 9, 3, 2), (2, 5, 1, 0, 4, 3)),
+         ((4341, 7, 3, 4, 8), (0, 2, 4, 3, 1)), ((2, 3, 2, 3, 2, 3, 2, 3, 5, 3, 2), (0, 2, 1, 4, 3, 6, 5, 8, 7, 10, 9))]
+
+
+def _check(shape, mapper, dtype, first):
+    """`first`: the tensor starts that many elements into its buffer (0: aligned, 1: not)."""
+    import cytnx_b200 as c
+
+    n = int(np.prod(shape))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    if dtype == torch.bool:
+        x = torch.randint(0, 2, (n + 1,), device="cuda", generator=g, dtype=torch.uint8).view(torch.bool)
+    elif dtype == torch.int16:
+        x = torch.randint(-30000, 30000, (n + 1,), device="cuda", generator=g, dtype=dtype)
+    else:
+        x = torch.randn(n + 1, dtype=dtype, device="cuda", generator=g)
+    x = x[first: first + n].view(*shape)
+    got = c.Tensor.from_torch(x).permute(list(mapper)).contiguous().to_torch()
+    assert torch.equal(got, x.permute(*mapper))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape,mapper", CASES)
+def test_short_neighbours(shape, mapper, dtype):
+    _check(shape, mapper, dtype, 0)
+    _check(shape, mapper, dtype, 1)
+
+
+def test_more_elements_than_32_bit_indices():
+    _check((2 ** 29 + 7, 2, 2), (0, 2, 1), torch.bool, 1)
+
+
+@pytest.mark.parametrize("dtype", [torch.bool, torch.float64])
+def test_seeded_shapes(dtype):
+    rng = np.random.default_rng(3)
+    for _ in range(60):
+        rank = int(rng.integers(3, 7))
+        shape = [int(v) for v in rng.choice([2, 2, 3, 4, 5, 7, 8, 9, 12, 17], rank)]
+        shape[int(rng.integers(rank))] = int(rng.integers(50, 900))
+        mapper = rng.permutation(rank)
+        _check(tuple(shape), tuple(int(m) for m in mapper), dtype, int(rng.integers(2)))
