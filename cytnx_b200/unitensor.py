@@ -87,6 +87,9 @@ class _LRU(dict):
 
 
 _PLANS: Dict[tuple, object] = _LRU(512)
+# permutations keep to themselves: a sweep over many layouts must not push out contraction plans, whose
+# device tables cost a synchronisation to make again
+_PERMUTES: Dict[tuple, object] = _LRU(512)
 
 
 class _ContractPlan:
@@ -403,10 +406,10 @@ class UniTensor:
             return UniTensor._new_dense(self._block.contiguous(), self._bonds, self._labels, self._rowrank,
                                         self._name, self._is_diag)
         require_cuda(self._data, "UniTensor::contiguous")
-        key = ("permute", id(self._layout), tuple(self._mapper), self._data.dtype)
-        plan = _PLANS.get(key)
+        key = (id(self._layout), tuple(self._mapper), self._data.dtype)
+        plan = _PERMUTES.get(key)
         if plan is None:
-            plan = _PLANS[key] = _PermutePlan(self)
+            plan = _PERMUTES[key] = _PermutePlan(self)
         lay_new = plan.layout
         out = torch.empty(lay_new.nelem, dtype=self._data.dtype, device=self._data.device)
         _lib.check(_lib.lib().ctn_permute_plan_run(plan.h, self._data.data_ptr(), out.data_ptr(), _lib.stream_ptr()),
