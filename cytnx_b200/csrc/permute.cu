@@ -406,6 +406,13 @@ constexpr int BLOCK_BATCH_SMALL = 40;
 // larger tiles of a single tensor move 6.4 instead of 5.4 TB/s
 constexpr int64_t BLOCK_OWN_BYTES = 8 << 20;
 
+// times a block's elements that its tiles may hold before it is copied element by element, the output
+// contiguous and the input read where it lies (short innermost axes that are each other's neighbours: a warp
+// then reads whole lines all the same).  60 f64 blocks, tiles / elements: [60,50,2,2] (0,1,3,2), 256 times, 448 /
+// 5.8 us; [100,12,12] (0,2,1), 7 times, 17.6 / 7.4; [100,16,16], 4 times, 17.8 / 10.9; [100,24,24], 1.8 times,
+// 18.1 / 18.7.
+constexpr int BLOCK_SPARSE = 3;
+
 template <int N>
 struct BlockBatch {
   int32_t n;
@@ -439,14 +446,14 @@ __global__ void __launch_bounds__(TILE_THREADS) k_permute_blocks(const T *__rest
   const TilePerm<BLOCK_RANK, uint32_t> &g = bb.p[lo];
   const uint32_t t = tile - bb.tile0[lo];
   switch (g.log_ta) {
-    case 0: {  // rows of ext[0] elements (the whole block when no axis moves); na elements in all
+    case 0: {  // element by element: ext[0] along the output's innermost axis, n_x axes outside it; na in all
       constexpr int PER = TILE_SMALL / TILE_THREADS;
       T v[PER];
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         const uint32_t u = t * TILE_SMALL + threadIdx.x + i * TILE_THREADS;
         if (u >= g.na) break;
-        uint32_t row = g.n_x ? u / g.ext[0] : 0, in = u - row * g.ext[0];
+        uint32_t row = g.n_x ? u / g.ext[0] : 0, in = (u - row * g.ext[0]) * g.ins[0];
         for (int k = 1; k <= g.n_x; ++k) {
           const uint32_t q = k < g.n_x ? row / g.ext[k] : 0;
           in += (row - q * g.ext[k]) * g.ins[k];
@@ -1108,19 +1115,19 @@ ctn_status block_permute_create(int dtype, int rank, int64_t nblocks, const uint
       out_stride_of_old[rmap[i]] = acc;
       acc *= rshape[rmap[i]];
     }
-    int64_t tiles;
-    if (r <= 1 || rmap[r - 1] == r - 1) {  // rows keep their order: copied in runs
+    int64_t tiles = 0;
+    const bool moves = r > 1 && rmap[r - 1] != r - 1;
+    if (moves) tiles = tile_geometry((int)es, TILE_SMALL, 16, r, rshape, rmap, in_stride, out_stride_of_old, g);
+    if (!moves || tiles * TILE_SMALL > BLOCK_SPARSE * n) {  // rows that keep their order, or tiles mostly empty
       g.log_ta = 0;
       g.na = (uint32_t)n;
-      g.ext[0] = (uint32_t)(r >= 1 ? rshape[r - 1] : 1);
       g.n_x = (int8_t)std::max(0, r - 1);
-      for (int k = 1; k < r; ++k) {  // outer axes, innermost of the output first
+      g.ext[0] = g.ins[0] = 1;
+      for (int k = 0; k < r; ++k) {  // innermost of the output first
         g.ext[k] = (uint32_t)rshape[rmap[r - 1 - k]];
         g.ins[k] = (uint32_t)in_stride[rmap[r - 1 - k]];
       }
       tiles = (n + TILE_SMALL - 1) / TILE_SMALL;
-    } else {
-      tiles = tile_geometry((int)es, TILE_SMALL, 16, r, rshape, rmap, in_stride, out_stride_of_old, g);
     }
     g.src = src_offs[b];
     g.dst = dst_offs[b];

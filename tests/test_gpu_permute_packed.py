@@ -55,3 +55,29 @@ def test_seeded_shapes(dtype):
         shape[int(rng.integers(rank))] = int(rng.integers(50, 900))
         mapper = rng.permutation(rank)
         _check(tuple(shape), tuple(int(m) for m in mapper), dtype, int(rng.integers(2)))
+
+
+# ---------------------------------------------------------------- many blocks in one launch
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("legs,mapper", [((2, 2), (0, 1, 3, 2)), ((3, 5), (1, 0, 3, 2)), ((12, 13), (0, 1, 3, 2)),
+                                         ((2, 7), (0, 3, 2, 1)), ((3, 2), (2, 3, 0, 1))])
+def test_blocks_with_short_neighbours(legs, mapper, dtype):
+    """Blocks that are copied element by element beside blocks that go in tiles, and one with a launch of its own."""
+    from cytnx_b200 import _lib
+    from cytnx_b200.core import Type
+
+    shapes = [(1, 1) + legs, (1, 9) + legs, (7, 5) + legs, (60, 51) + legs, (3, 2, 70, 65), (33, 2, 2, 40), (700, 701) + legs]
+    sizes = [int(np.prod(s)) for s in shapes]
+    offs = np.cumsum([1] + [n + 3 for n in sizes[:-1]]).astype(np.int64)
+    total = int(offs[-1]) + sizes[-1] + 5
+    g = torch.Generator(device="cuda")
+    g.manual_seed(2)
+    x = torch.randint(0, 2 if dtype == torch.bool else 30000, (total,), device="cuda", generator=g).to(dtype)
+    y, ref = torch.zeros_like(x), torch.zeros_like(x)
+    for s, n, o in zip(shapes, sizes, offs):
+        ref[o: o + n] = x[o: o + n].view(*s).permute(*mapper).reshape(-1)
+    shp, mp = np.array(shapes, dtype=np.uint64), np.array(mapper, dtype=np.uint64)
+    _lib.check(_lib.lib().ctn_permute_blocks(
+        x.data_ptr(), y.data_ptr(), Type.from_torch(dtype), 4, len(shapes), shp.ctypes.data_as(_lib.P_u64),
+        offs.ctypes.data_as(_lib.P_i64), offs.ctypes.data_as(_lib.P_i64), mp.ctypes.data_as(_lib.P_u64), _lib.stream_ptr()))
+    assert torch.equal(y, ref)
