@@ -489,9 +489,15 @@ __global__ void __launch_bounds__(TILE_THREADS) k_permute_blocks(const T *__rest
 // are faster).  NB bounds nb at compile time so the staging registers stay few (occupancy
 // carries the bytes in flight).
 constexpr int STAGED_THREADS = 256;
+// CTAs that the registers have to leave room for: without the bound the compiler took 58 registers instead of
+// 40 for bool and nb 7 ([7,5000000]: 30 us against 25)
+constexpr int staged_ctas(int es, int nb, int apt) {
+  const int words = nb * apt * (es > 4 ? es / 4 : 1);  // a thread's staged elements
+  return es <= 8 && words <= 16 ? (words <= 4 ? 8 : words <= 8 ? 7 : 6) : words <= 32 ? 4 : words <= 64 ? 2 : 1;
+}
 
 template <typename T, int NB, int APT, typename IT>
-__global__ void __launch_bounds__(STAGED_THREADS) k_transpose_staged(const T *__restrict__ src, T *__restrict__ dst,
+__global__ void __launch_bounds__(STAGED_THREADS, staged_ctas((int)sizeof(T), NB, APT)) k_transpose_staged(const T *__restrict__ src, T *__restrict__ dst,
                                                                      TransGeom g) {
   extern __shared__ __align__(16) unsigned char staged_smem[];
   T *tile = reinterpret_cast<T *>(staged_smem);
