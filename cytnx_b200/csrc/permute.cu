@@ -55,8 +55,9 @@ struct VecT<16> { using T = U128; };
 // input offset of a row takes a division per outer axis, so it is computed once per row of the
 // chunk, in parallel, into shared memory; a unit then takes one 32-bit division by the row length
 // (a multiply-high by floor(2^32 / d) with one correction) and a look-up, and a thread issues all
-// its loads before the first store.  PER = 1 (small tensors, where one unit's latency is all
-// there is) goes without the table.
+// its loads before the first store.  Without the table (every unit its own divisions): small tensors, one
+// unit a thread, where one unit's latency is all there is, and rows of a single unit, of which the table would
+// hold one entry each (int16 [33,24,4,1590,4] (2,3,0,1,4) 31.5 -> 25.6 us, f64 [1000000,3,2] (1,0,2) 17.6 -> 15.3).
 // Measured, a division per axis and unit -> this (read + written TB/s): f64 [2048,4,4,1024]
 // (0,2,1,3) 5.4 -> 6.6, [2047,5,3,1001] 3.0 -> 6.3; f32 [2047,5,3,1001] 1.5 -> 4.0; int16 0.8 ->
 // 2.8, bool 0.4 -> 1.4 (narrow odd rows: bound by the number of element accesses).  Assembling
@@ -64,6 +65,7 @@ struct VecT<16> { using T = U128; };
 // elements and up to 40 % slower for short rows of 8-byte elements.
 constexpr int ROW_THREADS = 256;
 constexpr int row_per(int unit) { return unit >= 16 ? 4 : unit >= 4 ? 8 : 16; }  // units per thread
+constexpr int ROW_PER_DIRECT = 4;                                                // without the table
 
 struct RowGeom {
   int n;                    // outer axes
@@ -94,7 +96,7 @@ __device__ __forceinline__ int64_t row_offset(const RowGeom &g, int64_t row) {
   return off + row * g.ins[g.n - 1];
 }
 
-template <typename U, int PER>
+template <typename U, int PER, bool TABLE>
 __global__ void __launch_bounds__(ROW_THREADS) k_row_copy(const U *__restrict__ src, U *__restrict__ dst,
                                                           const __grid_constant__ RowGeom g, int64_t total) {
   extern __shared__ int64_t row_off[];
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_copy(const U *__restrict__ 
       col = x - q * len;
       return q;
     };
-    if (PER > 1) {
+    if (TABLE) {
       uint32_t last;
       const uint32_t rows = split(c0 + cnt - 1, last) + 1;
       for (uint32_t i = threadIdx.x; i < rows; i += ROW_THREADS) row_off[i] = row_offset(g, r0 + i);
@@ -123,7 +125,7 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_copy(const U *__restrict__ 
       if (e < cnt) {
         uint32_t col;
         const uint32_t r = split(c0 + e, col);
-        v[i] = src[(PER > 1 ? row_off[r] : row_offset(g, r0 + r)) + col];
+        v[i] = src[(TABLE ? row_off[r] : row_offset(g, r0 + r)) + col];
       }
     }
 #pragma unroll
@@ -131,21 +133,22 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_copy(const U *__restrict__ 
       const uint32_t e = threadIdx.x + i * ROW_THREADS;
       if (e < cnt) dst[c + e] = v[i];
     }
-    if (PER > 1) __syncthreads();  // the next chunk reuses the table
+    if (TABLE) __syncthreads();  // the next chunk reuses the table
   }
 }
 
 template <typename U>
 static void launch_rows(const void *src, void *dst, const RowGeom &g, int64_t total, int nsm, cudaStream_t st) {
   constexpr int PER = row_per((int)sizeof(U)), CHUNK = ROW_THREADS * PER;
-  if (total < (int64_t)nsm * CHUNK) {
-    k_row_copy<U, 1><<<(unsigned)((total + ROW_THREADS - 1) / ROW_THREADS), ROW_THREADS, 0, st>>>((const U *)src, (U *)dst, g,
-                                                                                             total);
-    return;
-  }
-  const size_t smem = (size_t)(CHUNK / std::max<int64_t>(1, g.row) + 2) * sizeof(int64_t);
-  const int64_t grid = std::min<int64_t>((total + CHUNK - 1) / CHUNK, (int64_t)1 << 30);
-  k_row_copy<U, PER><<<(unsigned)grid, ROW_THREADS, smem, st>>>((const U *)src, (U *)dst, g, total);
+  auto go = [&](auto kern, int per, size_t smem) {
+    const int64_t chunk = (int64_t)ROW_THREADS * per, grid = std::min<int64_t>((total + chunk - 1) / chunk, (int64_t)1 << 30);
+    kern<<<(unsigned)grid, ROW_THREADS, smem, st>>>((const U *)src, (U *)dst, g, total);
+  };
+  // small: below one chunk of the table's form an SM, or four where the rows are so short that it gains little
+  // (f64 [200,200,4,2] (2,0,1,3) 3.2 / 2.7 us; f32 [256,4,4,255] (0,2,1,3) 3.5 / 7.7)
+  if (total < (int64_t)nsm * CHUNK * (g.row <= 2 ? 4 : 1)) go(k_row_copy<U, 1, false>, 1, 0);
+  else if (g.row == 1) go(k_row_copy<U, ROW_PER_DIRECT, false>, ROW_PER_DIRECT, 0);
+  else go(k_row_copy<U, PER, true>, PER, (size_t)(CHUNK / g.row + 2) * sizeof(int64_t));
 }
 
 // ---------------------------------------------------------------- tiled transpose
