@@ -72,7 +72,7 @@ struct RowGeom {
   int64_t ext[kMaxRank];    // their extents, innermost first
   int64_t ins[kMaxRank];    // input strides (in units)
   int64_t row;              // units per row
-  uint32_t rec;             // floor(2^32 / row), 2^32 - 1 for one unit per row (rows below 2^31 units)
+  uint32_t rec;             // floor(2^32 / row), 2^32 - 1 for one unit per row
   int wide;                 // 64-bit row numbers
 };
 
@@ -96,7 +96,11 @@ __device__ __forceinline__ int64_t row_offset(const RowGeom &g, int64_t row) {
   return off + row * g.ins[g.n - 1];
 }
 
-template <typename U, int PER, bool TABLE>
+// rows of 2^31 units and more are a mode of their own: a chunk lies in at most two of them, and the columns
+// take 64 bits
+enum RowMode { ROW_DIRECT, ROW_TABLE, ROW_LONG };
+
+template <typename U, int PER, int MODE>
 __global__ void __launch_bounds__(ROW_THREADS) k_row_copy(const U *__restrict__ src, U *__restrict__ dst,
                                                           const __grid_constant__ RowGeom g, int64_t total) {
   extern __shared__ int64_t row_off[];
@@ -112,10 +116,13 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_copy(const U *__restrict__ 
       col = x - q * len;
       return q;
     };
-    if (TABLE) {
+    if (MODE == ROW_TABLE) {
       uint32_t last;
       const uint32_t rows = split(c0 + cnt - 1, last) + 1;
       for (uint32_t i = threadIdx.x; i < rows; i += ROW_THREADS) row_off[i] = row_offset(g, r0 + i);
+      __syncthreads();
+    } else if (MODE == ROW_LONG) {
+      if (threadIdx.x < 2) row_off[threadIdx.x] = row_offset(g, r0 + threadIdx.x);
       __syncthreads();
     }
     U v[PER];
@@ -123,9 +130,14 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_copy(const U *__restrict__ 
     for (int i = 0; i < PER; ++i) {
       const uint32_t e = threadIdx.x + i * ROW_THREADS;
       if (e < cnt) {
-        uint32_t col;
-        const uint32_t r = split(c0 + e, col);
-        v[i] = src[(TABLE ? row_off[r] : row_offset(g, r0 + r)) + col];
+        if (MODE == ROW_LONG) {
+          const int64_t col = c - r0 * g.row + e;
+          v[i] = col < g.row ? src[row_off[0] + col] : src[row_off[1] + col - g.row];
+        } else {
+          uint32_t col;
+          const uint32_t r = split(c0 + e, col);
+          v[i] = src[(MODE == ROW_TABLE ? row_off[r] : row_offset(g, r0 + r)) + col];
+        }
       }
     }
 #pragma unroll
@@ -133,7 +145,7 @@ __global__ void __launch_bounds__(ROW_THREADS) k_row_copy(const U *__restrict__ 
       const uint32_t e = threadIdx.x + i * ROW_THREADS;
       if (e < cnt) dst[c + e] = v[i];
     }
-    if (TABLE) __syncthreads();  // the next chunk reuses the table
+    if (MODE != ROW_DIRECT) __syncthreads();  // the next chunk reuses the table
   }
 }
 
@@ -146,9 +158,10 @@ static void launch_rows(const void *src, void *dst, const RowGeom &g, int64_t to
   };
   // small: below one chunk of the table's form an SM, or four where the rows are so short that it gains little
   // (f64 [200,200,4,2] (2,0,1,3) 3.2 / 2.7 us; f32 [256,4,4,255] (0,2,1,3) 3.5 / 7.7)
-  if (total < (int64_t)nsm * CHUNK * (g.row <= 2 ? 4 : 1)) go(k_row_copy<U, 1, false>, 1, 0);
-  else if (g.row == 1) go(k_row_copy<U, ROW_PER_DIRECT, false>, ROW_PER_DIRECT, 0);
-  else go(k_row_copy<U, PER, true>, PER, (size_t)(CHUNK / g.row + 2) * sizeof(int64_t));
+  if (total < (int64_t)nsm * CHUNK * (g.row <= 2 ? 4 : 1)) go(k_row_copy<U, 1, ROW_DIRECT>, 1, 0);
+  else if (g.row == 1) go(k_row_copy<U, ROW_PER_DIRECT, ROW_DIRECT>, ROW_PER_DIRECT, 0);
+  else if (g.row < (int64_t)1 << 31) go(k_row_copy<U, PER, ROW_TABLE>, PER, (size_t)(CHUNK / g.row + 2) * sizeof(int64_t));
+  else go(k_row_copy<U, PER, ROW_LONG>, PER, 2 * sizeof(int64_t));
 }
 
 // ---------------------------------------------------------------- tiled transpose
@@ -952,17 +965,9 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
         break;
       }
     const int64_t unit = vb / ES, row = L / unit, total = n / unit;
-    // rows of 2^31 units and more: one more axis below them (the row is contiguous)
     RowGeom g;
     g.n = 0;
     g.row = row;
-    if (row >= ((int64_t)1 << 31)) {
-      int64_t part = 1 << 30;
-      while (row % part) part >>= 1;
-      g.ext[g.n] = row / part;
-      g.ins[g.n++] = part;
-      g.row = part;
-    }
     for (int i = r - 2; i >= 0; --i) {  // innermost outer axis first
       g.ext[g.n] = out_shape[i];
       g.ins[g.n++] = in_stride[rmap[i]] / unit;  // exact: multiples of a row

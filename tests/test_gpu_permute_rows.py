@@ -34,3 +34,11 @@ def test_short_rows(outer, mapper, row, dtype):
     shape, mapper = outer + (row,), mapper + (len(outer),)
     _check(shape, mapper, dtype, 0)
     _check(shape, mapper, dtype, 1)
+
+
+# single bytes (the buffer starts at an odd address): 2^32 units and more with 64-bit row numbers; rows of more
+# than 2^31 units, odd, whose ends fall inside a chunk; a row that no power of two divides, behind two axes
+@pytest.mark.parametrize("shape,mapper", [((3, 2, 715827885), (1, 0, 2)), ((2, 2, 2 ** 31 + 17), (1, 0, 2)),
+                                          ((2, 3, 2 ** 31 + 4096), (1, 0, 2))])
+def test_more_units_than_32_bits_count(shape, mapper):
+    _check(shape, mapper, torch.bool, 1)
