@@ -82,6 +82,7 @@ _SIGS = {
     "ctn_selftest_wait_timeout": (c_int, [c_int, ctypes.c_longlong, c_vp]),
     "ctn_selftest_barrier_timeout": (c_int, [ctypes.c_longlong, c_vp]),
     "ctn_selftest_lanczos_timeout": (c_int, [ctypes.c_longlong, c_vp]),
+    "ctn_selftest_permute_timeout": (c_int, [c_vp]),
     "ctn_dot_f64": (c_int, [c_vp, c_vp, c_i64, c_vp, c_vp]),
     "ctn_nrm2_f64": (c_int, [c_vp, c_i64, c_vp, c_vp]),
     "ctn_axpy_f64": (c_int, [c_vp, c_vp, c_i64, c_vp, c_dbl, c_vp]),

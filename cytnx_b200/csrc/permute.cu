@@ -25,8 +25,10 @@
 // stride arrays per call, cuMovemem_gpu.cu:139-152).
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "ctn_common.h"
@@ -625,7 +627,8 @@ struct TmaGeom {
   int64_t bshape[3];  // batch extents (tensor-map order: innermost first)
   int64_t bout[3];    // their output strides (elements)
   int64_t out_stride_a;
-  int *err;
+  unsigned *err;      // host memory (tma_err_word)
+  long long spins;    // mbarrier probes of a tile's wait
 };
 
 __device__ __forceinline__ uint32_t smem32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -708,13 +711,14 @@ __global__ void __launch_bounds__(TMA_THREADS) k_transpose_tma(const __grid_cons
   IT t = blockIdx.x;
   if (threadIdx.x == 0 && t < total) issue(t, 0);
   uint32_t phase[2] = {0, 0};
-  for (int i = 0; t < total; ++i, t += gridDim.x) {
+  int i = 0;
+  for (; t < total; ++i, t += gridDim.x) {
     const int slot = i & 1;
     const IT tn = t + gridDim.x;
     if (threadIdx.x == 0) {
       if (tn < total) issue(tn, slot ^ 1);  // that buffer was released by the last __syncthreads
       bool ok = false;
-      for (long long k = 0; k < TMA_SPIN && !ok; ++k) {
+      for (long long k = 0; k < g.spins && !ok; ++k) {
         uint32_t r;
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -724,7 +728,7 @@ __global__ void __launch_bounds__(TMA_THREADS) k_transpose_tma(const __grid_cons
         ok = r != 0;
       }
       if (!ok) {
-        atomicCAS(g.err, 0, 1);
+        *g.err = 1u;  // seen by the host when the kernel has ended
         stop = 1;
       }
     }
@@ -777,10 +781,10 @@ __global__ void __launch_bounds__(TMA_THREADS) k_transpose_tma(const __grid_cons
     }
     __syncthreads();  // this buffer may be refilled
   }
-  // an early stop may leave the prefetched tile in flight: wait for it (bounded)
+  // an early stop leaves its tile's copy in flight, and the next one's if it was issued: wait for them (bounded)
   if (threadIdx.x == 0 && stop) {
     for (int s2 = 0; s2 < 2; ++s2)
-      for (long long k = 0; k < TMA_SPIN; ++k) {
+      for (long long k = 0; k < TMA_SPIN && (s2 == (i & 1) || t + gridDim.x < total); ++k) {
         uint32_t r;
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -792,24 +796,46 @@ __global__ void __launch_bounds__(TMA_THREADS) k_transpose_tma(const __grid_cons
   }
 }
 
-static int *tma_err_word() {
-  static int *w = nullptr;
-  static int dev_of = -1;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!w || dev_of != dev) {
-    if (cudaMalloc(&w, sizeof(int)) != cudaSuccess) return nullptr;
-    cudaMemset(w, 0, sizeof(int));
-    dev_of = dev;
+// The word that a wait which ran out raises: 4 bytes of pinned host memory for the life of the process, which
+// every device can write, so the host sees it without a copy or a synchronisation.  Made on first use, also
+// under a stream capture (an allocation is legal there in the relaxed mode), by one thread.
+static std::atomic<unsigned *> tma_word{nullptr};
+static unsigned *tma_err_word() {
+  unsigned *w = tma_word.load(std::memory_order_acquire);
+  if (w) return w;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  if ((w = tma_word.load(std::memory_order_acquire))) return w;
+  void *p = nullptr;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+  const cudaError_t e = cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
   }
+  w = static_cast<unsigned *>(p);
+  *w = 0;
+  tma_word.store(w, std::memory_order_release);
   return w;
+}
+// CTN_ERR_TIMEOUT, once, after a permutation that gave up (asynchronously, like any launch's error)
+static ctn_status tma_status() {
+  unsigned *w = tma_word.load(std::memory_order_acquire);
+  if (w && *(volatile unsigned *)w && __atomic_exchange_n(w, 0u, __ATOMIC_RELAXED)) {
+    set_error("ctn_permute: an earlier permutation gave up waiting for a staged tile; its output is incomplete");
+    return CTN_ERR_TIMEOUT;
+  }
+  return CTN_OK;
 }
 
 // TMA path for the transpose case; returns false (nothing launched) when the geometry
 // does not fit a tensor map
 template <int ES>
 static bool try_transpose_tma(const void *src, void *dst, int r, const int64_t *rshape, const int *rmap,
-                              const int64_t *in_stride, const int64_t *out_stride, cudaStream_t st, ctn_status *res) {
+                              const int64_t *in_stride, const int64_t *out_stride, cudaStream_t st, ctn_status *res,
+                              long long spins = TMA_SPIN) {
   constexpr int TA = 128 / ES;
   const int a = r - 1, b = rmap[r - 1];
   if (r - 2 > 3) return false;
@@ -850,6 +876,7 @@ static bool try_transpose_tma(const void *src, void *dst, int r, const int64_t *
   if (g.tiles_a * g.tiles_b * g.batch > (1ll << 40)) return false;
   g.err = tma_err_word();
   if (!g.err) return false;
+  g.spins = spins;
   CUtensorMap map;
   const cuuint32_t box[5] = {(cuuint32_t)TA, (cuuint32_t)TMA_TB, 1, 1, 1};
   const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
@@ -1055,6 +1082,7 @@ static ctn_status permute_impl(const void *src, void *dst, int dtype, int rank,
                                const uint64_t *old_shape, const uint64_t *mapper, cudaStream_t st) {
   const size_t es = ctn_dtype_size(dtype);
   CTN_REQUIRE(es != 0, "ctn_permute: unknown dtype %d", dtype);
+  CTN_TRY(tma_status());
   CTN_REQUIRE(rank >= 0 && rank <= kMaxRank, "ctn_permute: rank %d out of range", rank);
   bool seen[kMaxRank] = {false};
   for (int i = 0; i < rank; ++i) {
@@ -1074,6 +1102,23 @@ static ctn_status permute_impl(const void *src, void *dst, int dtype, int rank,
   }
   set_error("ctn_permute: unsupported element size");
   return CTN_ERR_UNSUPPORTED;
+}
+
+// one int16 transpose whose waits give up at once
+static ctn_status selftest_tma_timeout(cudaStream_t st) {
+  const int64_t n = 1024, shape[2] = {n, n}, stride[2] = {n, 1};
+  const int rmap[2] = {1, 0};
+  CTN_TRY(tma_status());
+  char *buf = nullptr;
+  CTN_CUDA(cudaMalloc(&buf, 4 * n * n));
+  ctn_status rc = CTN_OK;
+  const bool launched = try_transpose_tma<2>(buf, buf + 2 * n * n, 2, shape, rmap, stride, stride, st, &rc, 0);
+  if (cudaStreamSynchronize(st) != cudaSuccess && rc == CTN_OK) rc = CTN_ERR_CUDA;
+  cudaFree(buf);
+  CTN_TRY(rc);
+  CTN_TRY(tma_status());
+  set_error(launched ? "ctn_selftest_permute_timeout: nothing was reported" : "ctn_selftest_permute_timeout: no tensor maps here");
+  return launched ? CTN_ERR_INVALID : CTN_ERR_UNSUPPORTED;
 }
 
 struct BlockPermute {
@@ -1179,6 +1224,7 @@ static ctn_status launch_batches(const BlockPermute &p, const void *src, void *d
 }
 
 ctn_status block_permute_run(const BlockPermute &p, const void *src, void *dst, cudaStream_t st) {
+  CTN_TRY(tma_status());
   for (const auto &o : p.own)
     CTN_TRY(permute_impl((const char *)src + o.src * p.es, (char *)dst + o.dst * p.es, p.dtype, p.rank, o.shape.data(),
                          p.mapper.data(), st));
@@ -1199,6 +1245,8 @@ extern "C" ctn_status ctn_permute(const void *src, void *dst, int dtype, int ran
                                   const uint64_t *old_shape, const uint64_t *mapper, void *stream) {
   return ctn::permute_impl(src, dst, dtype, rank, old_shape, mapper, ctn::as_stream(stream));
 }
+
+extern "C" ctn_status ctn_selftest_permute_timeout(void *stream) { return ctn::selftest_tma_timeout(ctn::as_stream(stream)); }
 
 extern "C" ctn_status ctn_permute_blocks(const void *src, void *dst, int dtype, int rank,
                                          int64_t nblocks, const uint64_t *old_shapes,

@@ -93,7 +93,9 @@ size_t ctn_dtype_size(int dtype);
 
 /* ---------------------------------------------------------------- permute
  * dst[new] = src[old] with new_shape[i] = old_shape[mapper[i]] (row-major);
- * bit-exact for every dtype.  rank <= 16.  src and dst must not overlap. */
+ * bit-exact for every dtype.  rank <= 16.  src and dst must not overlap.  A staged transpose
+ * whose bounded wait ran out is reported like any asynchronous error: the next permutation of the
+ * process returns CTN_ERR_TIMEOUT, once. */
 ctn_status ctn_permute(const void *src, void *dst, int dtype, int rank, const uint64_t *old_shape,
                        const uint64_t *mapper, void *stream);
 
@@ -225,6 +227,10 @@ ctn_status ctn_selftest_barrier_timeout(long long spin_limit, void *stream);
 /* The same for the step of ctn_lanczos_gnd, through its driver with the next iteration queued ahead: the
  * driver sees the error word, waits for what it has queued and returns CTN_ERR_TIMEOUT. */
 ctn_status ctn_selftest_lanczos_timeout(long long spin_limit, void *stream);
+/* The same for the TMA-staged transpose of ctn_permute: its waits give up at once, its copies in flight are
+ * waited for all the same, and the status that the next permutation of the process would return, once, is
+ * returned here: CTN_ERR_TIMEOUT. */
+ctn_status ctn_selftest_permute_timeout(void *stream);
 
 /* ---------------------------------------------------------------- BLAS-1 (FP64)
  * Results of reductions land in device memory (out points to device doubles). */
