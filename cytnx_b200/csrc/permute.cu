@@ -1051,7 +1051,20 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
   // tiles that are mostly empty (short axes that are each other's neighbours, which neither group can join)
   // give way to boxes over any axes
   auto packed = [&](int64_t ntiles, int cap) {
-    return permute_packed(ES, src, dst, r, rshape, rmap, in_stride, out_stride_of_old, n, ntiles * cap, nsm, st);
+    if (n >= nsm * PACK_MIN_PER_SM)
+      return permute_packed(ES, src, dst, r, rshape, rmap, in_stride, out_stride_of_old, n, ntiles * cap, nsm, st);
+    if ((double)ntiles * cap < PACK_RATIO * (double)n) return false;
+    RowGeom g;  // few elements: each a row of its own
+    g.n = r;
+    g.row = 1;
+    g.rec = 0xFFFFFFFFu;
+    g.wide = 0;
+    for (int i = 0; i < r; ++i) {
+      g.ext[i] = out_shape[r - 1 - i];
+      g.ins[i] = in_stride[rmap[r - 1 - i]];
+    }
+    launch_rows<T>(src, dst, g, n, nsm, st);
+    return true;
   };
   // 32-bit index arithmetic (a division costs several times less) when every offset fits
   if (n < ((int64_t)1 << 31)) {

@@ -27,13 +27,7 @@ namespace ctn {
 constexpr int PACK_THREADS = 256;
 constexpr int pack_per(int es) { return es >= 16 ? 4 : 8; }     // elements per thread
 constexpr int pack_ctas(int es) { return es == 8 ? 2 : 3; }     // resident CTAs per SM (registers)
-constexpr int PACK_PER_SMALL = 2;  // tensors with too few boxes to fill the SMs
 constexpr int PACK_WHOLE = 1 << 30;
-// Boxes are taken where the tiles would hold this many times their slots: above it they won in every one of 60
-// drawn shapes (f64 [200000,24,24], 3.4 times: 334 against 537 us), between 1 and 3.2 they lost more often than
-// not (f64 [8000,65,65], 2.2 times: 239 against 120 us), a box being cut at the ends of two axes and its offsets
-// being one register apiece.
-constexpr double PACK_RATIO = 3.3;
 
 // x / d for x below 2^16 and d from 2 to 2^16 / 2: the high word of x * (2^32 / d + 1)
 struct SmallDiv {
@@ -285,7 +279,6 @@ static bool packed(const void *src, void *dst, int r, const int64_t *rshape, con
   constexpr int PER = pack_per(ES), CTAS = pack_ctas(ES);
   auto go = [&](auto launch) { return launch(src, dst, r, rshape, rmap, in_stride, out_stride_of_old, tile_slots, nsm, st); };
   if (n >= (int64_t)1 << 31) return go(launch_packed<T, ES, PER, CTAS, uint64_t>);
-  if (n < (int64_t)nsm * 2 * PACK_THREADS * PER) return go(launch_packed<T, ES, PACK_PER_SMALL, 8, uint32_t>);
   return go(launch_packed<T, ES, PER, CTAS, uint32_t>);
 }
 
