@@ -87,7 +87,7 @@ struct ctn_heff2_plan {
   // split-precision state per kind (0: 3xTF32, 1: BF16x3)
   ctn::HeffSplit *split[2] = {nullptr, nullptr};
   int split_bn[2][2] = {{0, 0}, {0, 0}};          // tile widths of steps 1 and 4 per split kind (0: by size)
-  int split_epi[2][2] = {{-1, -1}, {-1, -1}};     // epilogue form per GEMM: -1 automatic, 0 direct, 1 staged
+  int split_epi[2][2] = {{-1, -1}, {-1, -1}};     // epilogue form per GEMM: -1 automatic, 0 direct, 1 staged, 2 fragments
   bool split_bound[2] = {false, false};
   ~ctn_heff2_plan() {
     for (auto *s : split) ctn::heff_split_free(s);

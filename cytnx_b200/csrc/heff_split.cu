@@ -358,9 +358,10 @@ ctn_status heff_split_prepare(ctn_heff2_plan *p, int kind) {
   for (size_t l = 0; l < p->Lb.size(); ++l) Lg[p->Lb[l].q[1]].push_back((int64_t)l);
   for (size_t q = 0; q < p->Pb.size(); ++q) Pg[p->Pb[q].q[0]].push_back((int64_t)q);
   // tile widths nobody has set: step 1 (short K, all columns of a sector side by side) takes 256
-  // columns when that leaves four tiles a worker, so that the last round stays a small part (D=4096
-  // bf16x3 38.9 -> 33.5 us, 3xTF32 59 -> 47 us; at D=2048, little more than one tile a worker, 128
-  // columns: bf16x3 15.5 us against 16.4); step 4 (long K, one sector's columns) takes 128
+  // columns where that leaves four tiles a worker (whole matvec, 128 -> 256 columns: XXZ D=4096 bf16x3 114 ->
+  // 108 us, 3xTF32 178 -> 166; Hubbard D=4000, 5.4 tiles a worker, 110 -> 108).  With fewer it hangs on how
+  // the last round falls: XXZ D=2500 to 4000 gains 3 to 10 %, Hubbard D=3000, 3.7 tiles a worker, loses 11 %
+  // (78 -> 88), and at D=2048 bf16x3 loses 2 %.  Step 4 (long K, one sector's columns) takes 128.
   int w1 = p->split_bn[kind][0], w4 = p->split_bn[kind][1];
   if (w1 == 0) {
     int64_t tiles = 0;
@@ -372,7 +373,7 @@ ctn_status heff_split_prepare(ctn_heff2_plan *p, int kind) {
       for (int64_t q : jt->second) N += p->Pb[q].d[1] * p->Pb[q].d[2] * p->Pb[q].d[3];
       tiles += (M + TC_BM - 1) / TC_BM * ((N + 255) / 256);
     }
-    w1 = tiles >= 4 * 148 ? 256 : 128;
+    w1 = tiles >= 4 * nsm_count() ? 256 : 128;
   }
   if (w4 == 0) w4 = 128;
   s->g1.set_width(w1);

@@ -294,8 +294,8 @@ void ctn_heff2_plan_destroy(ctn_heff2_plan *plan);
  * operand panels depend on the widths), so call ctn_heff2_set_env again.  Used by the
  * autotuner (TwoSiteHeff.autotune). */
 ctn_status ctn_heff2_set_tiles(ctn_heff2_plan *plan, int precision, int bn_step1, int bn_step4);
-/* epilogue form of the step-1 / step-4 tensor-core GEMMs: -1 automatic (staged through
- * shared memory when the tiles are at least half filled), 0 direct
+/* epilogue form of the step-1 / step-4 tensor-core GEMMs: -1 automatic (when the tiles are at
+ * least half filled staged through shared memory, or fragments for row-mapped outputs), 0 direct
  * (each lane stores its own accumulator row), 1 staged (whole row segments per store),
  * 2 fragments (16-lane TMEM fragments stored from registers, no shared memory; the 2-CTA
  * tiles run 2 as 1).  Takes effect on the next matvec; used by the autotuner. */

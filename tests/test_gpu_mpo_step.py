@@ -32,7 +32,7 @@ def test_mpo_step_from_a_misaligned_workspace(D):
 
 @pytest.mark.parametrize("prec,bound", [("3xtf32", 1e-5), ("bf16x3", 2e-3)])
 def test_widths_by_size_equal_the_set_ones(prec, bound):
-    """Step 1 at D=4096 takes 256 columns by itself: bitwise the widths a caller would set."""
+    """The widths taken by size give bitwise what a caller gets who sets them (which widths: test_split_widths)."""
     psi, H = two_site(4096)
     x = psi.flat_view()
     y, z, y64 = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x)
