@@ -6,7 +6,7 @@
 // src/BlockUniTensor.cpp:1180-1223) or one Gemm_Batch group entry (MKL build,
 // :1114-1177) per block pair; the reference's GPU Gemm_Batch is a serial loop of
 // cublasDgemm calls (src/backend/linalg_internal_gpu/cuGemm_Batch_internal.cu:23-64).
-// Here a CTA owns one 64x32 or 32x32 tile of one output block and walks the whole K range of
+// Here a CTA owns one tile (64x64, 64x32 or 32x32) of one output block and walks the whole K range of
 // all its pairs, so every output element is written exactly once (no atomics, no
 // zero-fill pass; tasks with no pair write zeros, matching Init's zeros blocks).
 // Operands are read in place from the block storage with per-pair leading
@@ -22,7 +22,7 @@
 namespace ctn {
 
 namespace {
-constexpr int BK = 16;  // k depth of a stage; tiles are BM x BN = 64 x 32 or 32 x 32
+constexpr int BK = F64_BK;  // k depth of a stage; tiles are BM x BN = 64 x 64, 64 x 32 or 32 x 32
 constexpr int PAD = 4;
 constexpr int NTHREADS = 128;
 
@@ -104,9 +104,9 @@ struct SliceCursor {
   }
 };
 
-// Each of the 4 warps computes a (BM / 2) x (BN / 2) quarter of the tile: 64 x 32 tiles 2 x 2
-// m16n8 products per k step, 32 x 32 tiles (plans of small blocks, where 64 rows are mostly
-// padding) 1 x 2.  Bound by the DMMA pipe, which runs at 128 cycles a product and SM quarter, and by
+// Each of the 4 warps computes a (BM / 2) x (BN / 2) quarter of the tile: 64 x 64 tiles 2 x 4
+// m16n8 products per k step, 64 x 32 tiles 2 x 2, 32 x 32 tiles (plans of small blocks, where 64 rows are
+// mostly padding) 1 x 2.  Bound by the DMMA pipe, which runs at 128 cycles a product and SM quarter, and by
 // how well the other warps' instructions hide behind it.  Two-site FP64 matvec, with the loads'
 // arithmetic inside the stage and 64 x 64 tiles -> this: D=4096 635 -> 555 us, D=3000 283 -> 249,
 // D=2048 126 -> 105, D=1500 61 -> 52, D=1024 33.0 -> 31.8.  Warps with tiles and stages of their own, which
@@ -323,7 +323,8 @@ ctn_status launch_gemm(const double *A, const double *B, double *C, const GemmTa
 }
 template <bool TA, bool TB>
 ctn_status launch_tiles(const double *A, const double *B, double *C, const GemmTaskD *d_tasks, const GemmPairD *d_pairs,
-                        const GemmTileD *d_tiles, int64_t ntiles, int bm, int nsm, cudaStream_t st) {
+                        const GemmTileD *d_tiles, int64_t ntiles, int bm, int bn, int nsm, cudaStream_t st) {
+  if (bn == 64) return launch_gemm<TA, TB, 64, 64>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, nsm, st);
   if (bm == 32) return launch_gemm<TA, TB, 32, 32>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, nsm, st);
   return launch_gemm<TA, TB, 64, 32>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, nsm, st);
 }
@@ -331,16 +332,16 @@ ctn_status launch_tiles(const double *A, const double *B, double *C, const GemmT
 
 ctn_status launch_gemm_f64(const double *A, const double *B, double *C, const GemmTaskD *d_tasks,
                            const GemmPairD *d_pairs, const GemmTileD *d_tiles, int64_t ntiles, int flags,
-                           int bm, cudaStream_t st) {
+                           int bm, int bn, cudaStream_t st) {
   if (ntiles == 0) return CTN_OK;
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   switch (flags & 3) {
-    case 0: return launch_tiles<false, false>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, nsm, st);
-    case 1: return launch_tiles<true, false>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, nsm, st);
-    case 2: return launch_tiles<false, true>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, nsm, st);
-    default: return launch_tiles<true, true>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, nsm, st);
+    case 0: return launch_tiles<false, false>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, bn, nsm, st);
+    case 1: return launch_tiles<true, false>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, bn, nsm, st);
+    case 2: return launch_tiles<false, true>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, bn, nsm, st);
+    default: return launch_tiles<true, true>(A, B, C, d_tasks, d_pairs, d_tiles, ntiles, bm, bn, nsm, st);
   }
 }
 

@@ -68,4 +68,15 @@ def test_scalar_times_vector(ta, tb):
 def test_tiles_with_remainders(ta, tb):
     sizes = [(1, 1, [3]), (31, 33, [16]), (32, 32, [15, 17]), (33, 31, [1, 0, 32]), (64, 32, [48]), (65, 97, [5, 7, 31]), (2, 70, []), (130, 3, [64])]
     _run(sizes, ta, tb)                               # small blocks: 32 x 32 tiles
-    _run([(256, 256, [40]), (320, 288, [16, 33])], ta, tb)  # little padding: 64 x 32 tiles
+    _run([(256, 256, [40]), (320, 288, [16, 33])], ta, tb)  # few tiles: 32 x 32 as well
+
+
+@pytest.mark.parametrize("ta", [False, True])
+@pytest.mark.parametrize("tb", [False, True])
+@pytest.mark.parametrize("m,n,ks", [(3000, 1000, [40, 7]),           # 64 x 32: 752 tiles of 64 x 64 are too few
+                                    (2040, 2043, [40, 17]),          # 64 x 64, remainders in every direction
+                                    (2048, 1985, [16, 3]),           # 64 x 64, two slices, one column in the last tile
+                                    (2040, 2043, [9]),               # one slice: 1024 tiles are too few, 64 x 32
+                                    (2945, 2999, [9]), (2945, 2999, [16])])  # 64 x 64 with one slice
+def test_wide_tiles(m, n, ks, ta, tb):
+    _run([(m, n, ks)], ta, tb)
