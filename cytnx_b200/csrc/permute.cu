@@ -1050,10 +1050,13 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
   constexpr int WANT = ES == 1 ? 128 : 64;
   // tiles that are mostly empty (short axes that are each other's neighbours, which neither group can join)
   // give way to boxes over any axes
-  auto packed = [&](int64_t ntiles, int cap) {
+  auto packed = [&](int64_t ntiles, int cap, int64_t na) {
+    // bytes whose tiles read runs of 16 and less: a warp's access takes a line for every few bytes, twice the
+    // slots' worth (bool [1653,8,2,1653,4] (0,2,4,3,1), tiles half full: 768 us, boxes 321; one thread per output row 452)
+    const int64_t slots = ntiles * cap * (ES == 1 && na <= 16 ? 2 : 1);
     if (n >= nsm * PACK_MIN_PER_SM)
-      return permute_packed(ES, src, dst, r, rshape, rmap, in_stride, out_stride_of_old, n, ntiles * cap, nsm, st);
-    if ((double)ntiles * cap < PACK_RATIO * (double)n) return false;
+      return permute_packed(ES, src, dst, r, rshape, rmap, in_stride, out_stride_of_old, n, slots, nsm, st);
+    if ((double)slots < PACK_RATIO * (double)n) return false;
     RowGeom g;  // few elements: each a row of its own
     g.n = r;
     g.row = 1;
@@ -1075,7 +1078,7 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
     // axes joined only where a group would be very short (a joined group needs an offset table)
     const bool small = ntiles < 2 * nsm;
     if (small) ntiles = tile_geometry(ES, TILE_SMALL, 16, r, rshape, rmap, in_stride, out_stride_of_old, g);
-    if (packed(ntiles, small ? TILE_SMALL : tile_cap(ES))) {
+    if (packed(ntiles, small ? TILE_SMALL : tile_cap(ES), (int64_t)g.na)) {
     } else if (small) {
       launch_tile<T, TILE_SMALL>(src, dst, g, ntiles, st);
     } else {
@@ -1085,7 +1088,7 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
     TilePerm<kMaxRank, uint64_t> g;
     g.src = g.dst = 0;
     const int64_t ntiles = tile_geometry(ES, tile_cap(ES), WANT, r, rshape, rmap, in_stride, out_stride_of_old, g);
-    if (!packed(ntiles, tile_cap(ES))) launch_tile<T, tile_cap(ES)>(src, dst, g, ntiles, st);
+    if (!packed(ntiles, tile_cap(ES), (int64_t)g.na)) launch_tile<T, tile_cap(ES)>(src, dst, g, ntiles, st);
   }
   CTN_CHECK_LAUNCH();
   return CTN_OK;

@@ -13,6 +13,7 @@ CASES = [((9, 2, 2), (0, 2, 1)), ((5000, 2, 2), (0, 2, 1)), ((5001, 3, 5), (0, 2
          ((300007, 2, 2), (0, 2, 1)), ((1201, 24, 24), (0, 2, 1)), ((7001, 10, 11), (0, 2, 1)),
          ((257, 131, 2, 3), (1, 0, 3, 2)), ((1009, 613, 2, 3), (1, 0, 3, 2)), ((300, 301, 4, 8), (1, 0, 3, 2)),
          ((601, 97, 4, 3), (3, 0, 2, 1)), ((601, 97, 4, 4, 3), (3, 1, 0, 4, 2)), ((1487, 4, 7, 16, 2), (0, 3, 1, 4, 2)),
+         ((165, 8, 2, 1653, 4), (0, 2, 4, 3, 1)), ((16, 9, 15101, 4), (3, 0, 2, 1)),  # bytes in runs of 4
          ((59, 16, 5, 16, 12, 8), (1, 2, 3, 0, 5, 4)), ((155, 155, 4, 9, 3, 2), (2, 5, 1, 0, 4, 3)),
          ((4341, 7, 3, 4, 8), (0, 2, 4, 3, 1)), ((2, 3, 2, 3, 2, 3, 2, 3, 5, 3, 2), (0, 2, 1, 4, 3, 6, 5, 8, 7, 10, 9))]
 
