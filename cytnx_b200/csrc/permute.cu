@@ -158,9 +158,10 @@ static void launch_rows(const void *src, void *dst, const RowGeom &g, int64_t to
     const int64_t chunk = (int64_t)ROW_THREADS * per, grid = std::min<int64_t>((total + chunk - 1) / chunk, (int64_t)1 << 30);
     kern<<<(unsigned)grid, ROW_THREADS, smem, st>>>((const U *)src, (U *)dst, g, total);
   };
-  // small: below one chunk of the table's form an SM, or four where the rows are so short that it gains little
-  // (f64 [200,200,4,2] (2,0,1,3) 3.2 / 2.7 us; f32 [256,4,4,255] (0,2,1,3) 3.5 / 7.7)
-  if (total < (int64_t)nsm * CHUNK * (g.row <= 2 ? 4 : 1)) go(k_row_copy<U, 1, ROW_DIRECT>, 1, 0);
+  // small: below one chunk of the table's form an SM, or two where the rows are so short that it gains little
+  // (f64 [200,200,4,2] (2,0,1,3) 3.2 / 2.7 us; f32 [256,4,4,255] (0,2,1,3) 3.5 / 7.7; at three of them, bool
+  // [203124,5,8] (1,0,2), one unit a thread is slower, 6.7 against 5.2)
+  if (total < (int64_t)nsm * CHUNK * (g.row <= 2 ? 2 : 1)) go(k_row_copy<U, 1, ROW_DIRECT>, 1, 0);
   else if (g.row == 1) go(k_row_copy<U, ROW_PER_DIRECT, ROW_DIRECT>, ROW_PER_DIRECT, 0);
   else if (g.row < (int64_t)1 << 31) go(k_row_copy<U, PER, ROW_TABLE>, PER, (size_t)(CHUNK / g.row + 2) * sizeof(int64_t));
   else go(k_row_copy<U, PER, ROW_LONG>, PER, 2 * sizeof(int64_t));
