@@ -10,6 +10,7 @@
 // result is complete in device memory when the kernel ends -- deterministic
 // summation order for a fixed grid.
 #include <algorithm>
+#include <mutex>
 
 #include "ctn_common.h"
 #include "blas1.cuh"
@@ -809,6 +810,35 @@ ctn_status lanczos_step_f64(const float *w, const double *u, const double *up, c
   return lanczos_step_any(w, u, up, q, dst, n, alpha, gamma, s, sp, nrm, ws, st);
 }
 
+// CTAs of a kernel with `threads` threads that are resident together per SM, and the SMs, of the current device: 0
+// CTAs without cooperative launch.  Asked once per device and kernel (a step runs hundreds of times per solve);
+// `slot` is the caller's table, written whole under its lock
+struct Resident {
+  std::mutex mu;
+  struct {
+    bool known = false;
+    int per_sm = 0, sms = 0;
+  } dev[64];
+};
+static ctn_status resident(Resident &slot, const void *kern, int *per_sm, int *sms) {
+  int dev = 0;
+  CTN_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(slot.mu);
+  auto &e = slot.dev[dev & 63];
+  if (!e.known) {
+    int coop = 0, nsm = 0, occ = 0;
+    CTN_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    CTN_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    CTN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, RT, 0));
+    e.per_sm = coop ? occ : 0;
+    e.sms = nsm;
+    e.known = true;
+  }
+  *per_sm = e.per_sm;
+  *sms = e.sms;
+  return CTN_OK;
+}
+
 // the fused step: one cooperative launch of k_krylov_step with k_dot2s's grid (capped at the
 // CTAs that fit on the device at once); CTN_ERR_UNSUPPORTED when the device has no
 // cooperative launch (the caller then runs the two kernels)
@@ -821,23 +851,11 @@ static ctn_status krylov_step_any(const WT *w, const double *u, const double *up
   void (*kern)(const WT *, const double *, const double *, const double *, double *, int64_t, const double *,
                const double *, double *, double *, double *, double *, double *, unsigned *, unsigned, long long) =
       vec ? k_krylov_step<true, WT> : k_krylov_step<false, WT>;
-  // resident CTAs of this kernel on the device (queried once per device: the step runs hundreds
-  // of times per solve); 0 = the device has no cooperative launch
-  static int resident[64][2];
-  static bool known[64][2];
-  int dev = 0;
-  CTN_CUDA(cudaGetDevice(&dev));
-  const int di = dev & 63;
-  if (!known[di][vec]) {
-    int coop = 0, nsm = 0, occ = 0;
-    CTN_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    CTN_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    CTN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, RT, 0));
-    resident[di][vec] = coop ? std::max(1, nsm * occ) : 0;
-    known[di][vec] = true;
-  }
-  if (resident[di][vec] == 0) return CTN_ERR_UNSUPPORTED;
-  const int g = std::min(grid_stream(n), resident[di][vec]);
+  static Resident slot[2];
+  int per_sm = 0, sms = 0;
+  CTN_TRY(resident(slot[vec], (const void *)kern, &per_sm, &sms));
+  if (per_sm == 0) return CTN_ERR_UNSUPPORTED;
+  const int g = std::min(grid_stream(n), per_sm * sms);
   void *args[] = {(void *)&w,   (void *)&u,         (void *)&up,        (void *)&q,   (void *)&dst,
                   (void *)&n,   (void *)&s,         (void *)&sp,        (void *)&out_alpha,
                   (void *)&out_gamma, (void *)&nrm, (void *)&ws,        (void *)&ws2, (void *)&err,
@@ -863,23 +881,12 @@ static ctn_status lanczos_gnd_step_any(const WT *w, const double *p1, const doub
   const bool vec = aligned16(w) && aligned16(p1) && aligned16(dst) && (!p0 || aligned16(p0));
   void (*kern)(const WT *, const double *, const double *, double *, int64_t, const double *, double *, double *,
                double *, unsigned *, unsigned, long long) = vec ? k_lanczos_gnd_step<true, WT> : k_lanczos_gnd_step<false, WT>;
-  // CTAs per SM that are resident together, queried once per device; 0 = no cooperative launch
-  static int per_sm[64][2], sms[64];
-  static bool known[64][2];
-  int dev = 0;
-  CTN_CUDA(cudaGetDevice(&dev));
-  const int di = dev & 63;
-  if (!known[di][vec]) {
-    int coop = 0, occ = 0;
-    CTN_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    CTN_CUDA(cudaDeviceGetAttribute(&sms[di], cudaDevAttrMultiProcessorCount, dev));
-    CTN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, RT, 0));
-    per_sm[di][vec] = coop ? occ : 0;
-    known[di][vec] = true;
-  }
-  if (per_sm[di][vec] == 0) return CTN_ERR_UNSUPPORTED;
+  static Resident slot[2];
+  int per_sm = 0, sms = 0;
+  CTN_TRY(resident(slot[vec], (const void *)kern, &per_sm, &sms));
+  if (per_sm == 0) return CTN_ERR_UNSUPPORTED;
   // at most three CTAs an SM: whole waves below GND_CTAS on 148 SMs
-  const int most = std::min(GND_CTAS, sms[di] * std::min(3, per_sm[di][vec]));
+  const int most = std::min(GND_CTAS, sms * std::min(3, per_sm));
   const int g = std::max(1, std::min(grid_stream(n), most));
   if (spins == 0) spins = BARRIER_SPINS;
   void *args[] = {(void *)&w,         (void *)&p1,       (void *)&p0, (void *)&dst, (void *)&n,    (void *)&beta,
