@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -1265,15 +1266,27 @@ extern "C" ctn_status ctn_permute(const void *src, void *dst, int dtype, int ran
 
 extern "C" ctn_status ctn_selftest_permute_timeout(void *stream) { return ctn::selftest_tma_timeout(ctn::as_stream(stream)); }
 
+// the descriptors' memory may not be there: a status, not an exception across the C boundary
+template <class F>
+static ctn_status no_throw(F f) {
+  try {
+    return f();
+  } catch (const std::exception &e) {
+    ctn::set_error("ctn_permute_blocks: %s", e.what());
+    return CTN_ERR_INVALID;
+  }
+}
+
 extern "C" ctn_status ctn_permute_blocks(const void *src, void *dst, int dtype, int rank,
                                          int64_t nblocks, const uint64_t *old_shapes,
                                          const int64_t *src_offs, const int64_t *dst_offs,
                                          const uint64_t *mapper, void *stream) {
-  ctn::BlockPermute *p = nullptr;
-  CTN_TRY(ctn::block_permute_create(dtype, rank, nblocks, old_shapes, src_offs, dst_offs, mapper, &p));
-  const ctn_status s = ctn::block_permute_run(*p, src, dst, ctn::as_stream(stream));
-  ctn::block_permute_destroy(p);
-  return s;
+  return no_throw([&]() -> ctn_status {
+    ctn::BlockPermute *p = nullptr;
+    CTN_TRY(ctn::block_permute_create(dtype, rank, nblocks, old_shapes, src_offs, dst_offs, mapper, &p));
+    const std::unique_ptr<ctn::BlockPermute, void (*)(ctn::BlockPermute *)> own(p, ctn::block_permute_destroy);
+    return ctn::block_permute_run(*p, src, dst, ctn::as_stream(stream));
+  });
 }
 
 struct ctn_permute_plan {
@@ -1285,10 +1298,12 @@ extern "C" ctn_status ctn_permute_plan_create(int dtype, int rank, int64_t nbloc
                                               const int64_t *src_offs, const int64_t *dst_offs,
                                               const uint64_t *mapper, ctn_permute_plan **plan) {
   CTN_REQUIRE(plan, "ctn_permute_plan_create: null argument");
-  std::unique_ptr<ctn_permute_plan> h(new ctn_permute_plan());
-  CTN_TRY(ctn::block_permute_create(dtype, rank, nblocks, old_shapes, src_offs, dst_offs, mapper, &h->p));
-  *plan = h.release();
-  return CTN_OK;
+  return no_throw([&]() -> ctn_status {
+    std::unique_ptr<ctn_permute_plan> h(new ctn_permute_plan());
+    CTN_TRY(ctn::block_permute_create(dtype, rank, nblocks, old_shapes, src_offs, dst_offs, mapper, &h->p));
+    *plan = h.release();
+    return CTN_OK;
+  });
 }
 extern "C" ctn_status ctn_permute_plan_run(const ctn_permute_plan *plan, const void *src, void *dst, void *stream) {
   CTN_REQUIRE(plan, "ctn_permute_plan_run: null plan");
