@@ -470,9 +470,10 @@ extern "C" ctn_status ctn_heff2_set_tiles(ctn_heff2_plan *p, int precision, int 
               "ctn_heff2_set_tiles: tile widths must be one of 32, 48, 64, 96, 128, 144, 160, 192, 256 "
               "or -128, -192, -256 (2-CTA tiles)");
   const int k = split_kind(precision);
-  if (p->split_bn[k][0] == bn_step1 && p->split_bn[k][1] == bn_step4) return CTN_OK;
   p->split_bn[k][0] = bn_step1;
   p->split_bn[k][1] = bn_step4;
+  // tables that have these widths, set or taken by size, stay, and their binding with them
+  if (ctn::heff_split_has_widths(p->split[k], bn_step1, bn_step4)) return CTN_OK;
   ctn::heff_split_free(p->split[k]);
   p->split[k] = nullptr;
   p->split_bound[k] = false;  // the panels depend on the tile widths: bind again

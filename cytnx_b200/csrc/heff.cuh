@@ -61,6 +61,7 @@ ctn_status heff_split_matvec(struct ::ctn_heff2_plan *p, int kind, const double 
 ctn_status heff_split_matvec_f32out(struct ::ctn_heff2_plan *p, int kind, const double *psi, float *out,
                                     cudaStream_t st);
 void heff_split_free(HeffSplit *s);
+bool heff_split_has_widths(const HeffSplit *s, int bn_step1, int bn_step4);  // false for null
 double heff_split_gemm_flops(const struct ::ctn_heff2_plan *p, int kind, int step);
 ctn_status heff_split_stats(const struct ::ctn_heff2_plan *p, int kind, double *out);
 void heff_split_apply_epilogue(struct ::ctn_heff2_plan *p, int kind);

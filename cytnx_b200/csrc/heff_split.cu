@@ -82,6 +82,9 @@ struct HeffSplit {
 };
 
 void heff_split_free(HeffSplit *s) { delete s; }
+bool heff_split_has_widths(const HeffSplit *s, int bn_step1, int bn_step4) {
+  return s && s->g1.width() == bn_step1 && s->g4.width() == bn_step4;
+}
 
 namespace {
 constexpr int KALIGN = 8;

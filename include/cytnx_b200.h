@@ -290,8 +290,9 @@ ctn_status ctn_heff2_split_stats(ctn_heff2_plan *plan, int precision, double *ou
 void ctn_heff2_plan_destroy(ctn_heff2_plan *plan);
 /* tile widths (N of the UMMA tiles: 32, 48, 64, 96, 128, 144, 160, 192 or 256; negative -128, -192,
  * -256 select 2-CTA cta_group::2 tiles of 256 rows) of the step-1 and
- * step-4 tensor-core GEMMs of a split precision; drops that precision's binding (the
- * operand panels depend on the widths), so call ctn_heff2_set_env again.  Used by the
+ * step-4 tensor-core GEMMs of a split precision; unless the plan has these widths already, drops
+ * that precision's binding (the operand panels depend on the widths), so call ctn_heff2_set_env
+ * again.  Used by the
  * autotuner (TwoSiteHeff.autotune). */
 ctn_status ctn_heff2_set_tiles(ctn_heff2_plan *plan, int precision, int bn_step1, int bn_step4);
 /* epilogue form of the step-1 / step-4 tensor-core GEMMs: -1 automatic (when the tiles are at
