@@ -13,8 +13,8 @@ TRANSPOSES = [((63, 65), (1, 0)), ((64, 129), (1, 0)), ((2, 5000), (1, 0)), ((50
               ((33, 3, 37, 130), (3, 1, 0, 2)), ((5, 700, 3), (2, 1, 0)), ((40, 30, 20), (2, 1, 0)),
               ((11, 2, 3, 2, 257), (4, 2, 0, 3, 1)), ((257, 129, 131), (2, 0, 1)), ((300, 40, 70, 3), (3, 1, 2, 0)),
               ((1500, 2, 2, 901), (3, 2, 1, 0))]
-# rows kept whole: shorter and longer than the 128 bytes where shifted vectors begin, of every
-# remainder class, and a last vector that reaches the end of the tensor
+# rows kept whole: of every remainder class of the 16-byte units, short and long, and a last unit that
+# reaches the end of the tensor
 ROWS = [((5, 7, 3), (1, 0, 2)), ((5, 7, 1), (1, 0, 2)), ((9, 4, 17), (1, 0, 2)), ((3, 5, 4, 129), (1, 2, 0, 3)),
         ((11, 2, 3, 131), (2, 0, 1, 3)), ((6, 5, 1001), (1, 0, 2)), ((2, 3, 2, 3, 64), (3, 1, 2, 0, 4)), ((700, 3, 37), (1, 0, 2))]
 
