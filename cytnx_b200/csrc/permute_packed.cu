@@ -27,6 +27,10 @@ namespace ctn {
 constexpr int PACK_THREADS = 256;
 constexpr int pack_per(int es) { return es >= 16 ? 4 : 8; }     // elements per thread
 constexpr int pack_ctas(int es) { return es == 8 ? 2 : 3; }     // resident CTAs per SM (registers)
+// elements of 4 bytes and less below this many an SM: two a thread, eight CTAs an SM (a box's latency is most of
+// the time: bool [5,16,17,25,25] (1,3,2,4,0) 8.6 -> 6.3 us, f32 [183,4,7,4,33] (1,3,0,4,2) 7.4 -> 5.9; 8-byte
+// elements, f64 [4000,20,20] (0,2,1), 6.7 -> 7.2)
+constexpr int64_t PACK_SMALL_PER_SM = 16384;
 constexpr int PACK_WHOLE = 1 << 30;
 
 // x / d for x below 2^16 and d from 2 to 2^16 / 2: the high word of x * (2^32 / d + 1)
@@ -279,6 +283,8 @@ static bool packed(const void *src, void *dst, int r, const int64_t *rshape, con
   constexpr int PER = pack_per(ES), CTAS = pack_ctas(ES);
   auto go = [&](auto launch) { return launch(src, dst, r, rshape, rmap, in_stride, out_stride_of_old, tile_slots, nsm, st); };
   if (n >= (int64_t)1 << 31) return go(launch_packed<T, ES, PER, CTAS, uint64_t>);
+  if constexpr (ES <= 4)
+    if (n < nsm * PACK_SMALL_PER_SM) return go(launch_packed<T, ES, 2, 8, uint32_t>);
   return go(launch_packed<T, ES, PER, CTAS, uint32_t>);
 }
 

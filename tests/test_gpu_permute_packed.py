@@ -8,13 +8,15 @@ pytestmark = pytest.mark.gpu
 DTYPES = [torch.bool, torch.int16, torch.float32, torch.float64, torch.complex128]
 # neighbours on both sides with the same axis behind them, on both sides with different ones, on one side only;
 # axes cut into equal and unequal chunks on either side and on both; one box; boxes of several axes; planes wider
-# than half a tile's side; few elements (512 a box) and many
+# than half a tile's side; few elements (one by one), more (512 a box up to 4 bytes) and many
 CASES = [((9, 2, 2), (0, 2, 1)), ((5000, 2, 2), (0, 2, 1)), ((5001, 3, 5), (0, 2, 1)), ((70001, 2, 3), (0, 2, 1)),
          ((300007, 2, 2), (0, 2, 1)), ((1201, 24, 24), (0, 2, 1)), ((7001, 10, 11), (0, 2, 1)),
          ((257, 131, 2, 3), (1, 0, 3, 2)), ((1009, 613, 2, 3), (1, 0, 3, 2)), ((300, 301, 4, 8), (1, 0, 3, 2)),
          ((601, 97, 4, 3), (3, 0, 2, 1)), ((601, 97, 4, 4, 3), (3, 1, 0, 4, 2)), ((1487, 4, 7, 16, 2), (0, 3, 1, 4, 2)),
          ((165, 8, 2, 1653, 4), (0, 2, 4, 3, 1)), ((16, 9, 15101, 4), (3, 0, 2, 1)),  # bytes in runs of 4
          ((59, 16, 5, 16, 12, 8), (1, 2, 3, 0, 5, 4)), ((155, 155, 4, 9, 3, 2), (2, 5, 1, 0, 4, 3)),
+         ((183, 4, 7, 4, 33), (1, 3, 0, 4, 2)), ((9, 8, 287, 31), (2, 0, 3, 1)), ((700, 700, 3, 2), (1, 0, 3, 2)),
+         ((2000, 24, 20), (0, 2, 1)), ((5, 16, 17, 125, 25), (1, 3, 2, 4, 0)),
          ((4341, 7, 3, 4, 8), (0, 2, 4, 3, 1)), ((2, 3, 2, 3, 2, 3, 2, 3, 5, 3, 2), (0, 2, 1, 4, 3, 6, 5, 8, 7, 10, 9))]
 
 
