@@ -59,8 +59,8 @@ struct VecT<16> { using T = U128; };
 // chunk, in parallel, into shared memory; a unit then takes one 32-bit division by the row length
 // (a multiply-high by floor(2^32 / d) with one correction) and a look-up, and a thread issues all
 // its loads before the first store.  Without the table (every unit its own divisions): small tensors, one
-// unit a thread, where one unit's latency is all there is, and rows of a single unit, of which the table would
-// hold one entry each (int16 [33,24,4,1590,4] (2,3,0,1,4) 31.5 -> 25.6 us, f64 [1000000,3,2] (1,0,2) 17.6 -> 15.3).
+// unit a thread, where one unit's latency is all there is, and elements that are rows of their own, of which
+// the table would hold one entry each.
 // Measured, a division per axis and unit -> this (read + written TB/s): f64 [2048,4,4,1024]
 // (0,2,1,3) 5.4 -> 6.6, [2047,5,3,1001] 3.0 -> 6.3; f32 [2047,5,3,1001] 1.5 -> 4.0; int16 0.8 ->
 // 2.8, bool 0.4 -> 1.4 (narrow odd rows: bound by the number of element accesses).  Assembling
@@ -160,8 +160,7 @@ static void launch_rows(const void *src, void *dst, const RowGeom &g, int64_t to
     kern<<<(unsigned)grid, ROW_THREADS, smem, st>>>((const U *)src, (U *)dst, g, total);
   };
   // small: below one chunk of the table's form an SM, or two where the rows are so short that it gains little
-  // (f64 [200,200,4,2] (2,0,1,3) 3.2 / 2.7 us; f32 [256,4,4,255] (0,2,1,3) 3.5 / 7.7; at three of them, bool
-  // [203124,5,8] (1,0,2), one unit a thread is slower, 6.7 against 5.2)
+  // (int16 [4,17,1323,16] (2,1,0,3) 3.4 / 2.7 us; f32 [256,4,4,255] (0,2,1,3) 3.5 / 7.7)
   if (total < (int64_t)nsm * CHUNK * (g.row <= 2 ? 2 : 1)) go(k_row_copy<U, 1, ROW_DIRECT>, 1, 0);
   else if (g.row == 1) go(k_row_copy<U, ROW_PER_DIRECT, ROW_DIRECT>, ROW_PER_DIRECT, 0);
   else if (g.row < (int64_t)1 << 31) go(k_row_copy<U, PER, ROW_TABLE>, PER, (size_t)(CHUNK / g.row + 2) * sizeof(int64_t));
@@ -994,6 +993,23 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
         break;
       }
     const int64_t unit = vb / ES, row = L / unit, total = n / unit;
+    // each row is one unit: a permutation of units, whose innermost axis moves, and a tiled transpose reads
+    // whole lines of them where a copy row by row takes a line for each (row copy -> this: int16
+    // [4,271049,24,2] (2,0,1,3) 272 -> 42 us, f64 [512,3,3,512,2] (3,1,2,0,4) 16.2 -> 9.6, f32 [2000,2000,4] (1,0,2)
+    // 31.4 -> 19.8); below 1024 units an SM the copy, one unit a thread (f64 [12,5746,2] (1,0,2) 3.6 -> 2.2)
+    if (row == 1 && total >= nsm * 1024) {
+      uint64_t ushape[kMaxRank], umap[kMaxRank];
+      for (int i = 0; i + 1 < r; ++i) {
+        ushape[i] = (uint64_t)rshape[i];
+        umap[i] = (uint64_t)rmap[i];
+      }
+      switch (vb) {
+        case 16: return launch_perm<16>(src, dst, r - 1, ushape, umap, st);
+        case 8: return launch_perm<8>(src, dst, r - 1, ushape, umap, st);
+        case 4: return launch_perm<4>(src, dst, r - 1, ushape, umap, st);
+        default: return launch_perm<2>(src, dst, r - 1, ushape, umap, st);
+      }
+    }
     RowGeom g;
     g.n = 0;
     g.row = row;
