@@ -1074,7 +1074,7 @@ static ctn_status launch_perm(const void *src, void *dst, int rank, const uint64
     const int64_t slots = ntiles * cap * (ES == 1 && na <= 16 ? 2 : 1);
     if (n >= nsm * PACK_MIN_PER_SM)
       return permute_packed(ES, src, dst, r, rshape, rmap, in_stride, out_stride_of_old, n, slots, nsm, st);
-    if ((double)slots < PACK_RATIO * (double)n) return false;
+    if ((double)slots < FEW_RATIO * (double)n) return false;
     RowGeom g;  // few elements: each a row of its own
     g.n = r;
     g.row = 1;

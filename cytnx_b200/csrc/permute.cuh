@@ -17,14 +17,11 @@ constexpr int tile_pitch(int es, int ta) {
   return es >= 4 ? (ta | 1) : es == 2 ? (ta % 4 == 0 ? ta + 2 : ta) : (ta % 8 == 0 ? ta + 4 : ta);
 }
 
-// Boxes over any axes are taken from this many elements an SM on, and where the tiles would hold this many times
-// their slots: above it they won in every one of 60 drawn shapes (f64 [200000,24,24], 3.4 times: 334 against
-// 537 us), between 1 and 3.2 they lost more often than not (f64 [8000,65,65], 2.2 times: 239 against 120 us), a
-// box being cut at the ends of two axes and its offsets being one register apiece.  Fewer elements go one by one,
-// whole rows of divisions but no set-up (f64 [256,256,2,2] (0,1,3,2) 3.5 -> 3.1 us, bool [7,151,17,31] (1,0,3,2) 6.6
-// -> 5.4; at [1000,1000,2,2], 27000 an SM, 18 against 12).
+// Boxes over any axes are taken from this many elements an SM on.  Fewer elements go one by one where the tiles
+// would hold more than FEW_RATIO times their slots: whole rows of divisions but no set-up (f64 [256,256,2,2]
+// (0,1,3,2) 3.5 -> 3.1 us, bool [7,151,17,31] (1,0,3,2) 6.6 -> 5.4; at [1000,1000,2,2], 27000 an SM, 18 against 12).
 constexpr int64_t PACK_MIN_PER_SM = 4096;
-constexpr double PACK_RATIO = 3.3;
+constexpr double FEW_RATIO = 3.3;
 
 // permute_packed.cu: a reduced permutation of rank r (axes merged, innermost moving; strides in elements, those
 // of the output by old axis) of n elements of `es` bytes, whose tiles would have tile_slots slots.  False,
